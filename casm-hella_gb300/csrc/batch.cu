@@ -162,6 +162,7 @@ struct hella_batch {
   hg::SmoothBeam *d_sbeams = nullptr;
   hg::GulpPos *d_pos = nullptr;
   std::vector<hg::DedispBeam> dbeams;
+  std::vector<float> taps;        // host copy of d_taps
   int items_dpt = -1;             // DM tile of the work-item prefix held in d_dbeams
   std::vector<uint8_t> keep;      // [nbeam][nchan] killmasks (1: channel summed)
   int4 *d_bmeta = nullptr;        // per-beam tile tables (beams that kill channels)
@@ -640,6 +641,7 @@ hg::SmoothArgs smooth_args(hella_batch *b, int w0, int nw) {
   a.taps = b->d_taps;
   a.tap_off = b->d_tapoff;
   a.tap_n = b->d_tapn;
+  a.taps_host = b->taps.data();
   a.snr = b->p.snr;
   a.nogate = b->p.always_find_peaks != 0;
   return a;
@@ -937,6 +939,7 @@ hella_status hella_batch_create(hella_batch **out, const hella_batch_params *bp)
   std::vector<float> taps;
   std::vector<int> toff, tn;
   hg::smoothing_taps(*p, z.nbox, &taps, &toff, &tn);
+  b->taps = taps;
   if ((s = dalloc(b, (void **)&b->d_taps, taps.size() * 4)) != HELLA_OK) return fail(s);
   if ((s = dalloc(b, (void **)&b->d_tapoff, toff.size() * 4)) != HELLA_OK) return fail(s);
   if ((s = dalloc(b, (void **)&b->d_tapn, tn.size() * 4)) != HELLA_OK) return fail(s);

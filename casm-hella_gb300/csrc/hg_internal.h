@@ -295,12 +295,9 @@ struct SmoothArgs {
   const int *tap_off;       // [nbox] offset into taps
   const int *tap_n;         // [nbox] padded tap count (multiple of 16)
   float snr;
-  int split;                // FIR: first width of the second width group
-                            // (w0 + nw: one group); set by smooth_planes
+  const float *taps_host;   // host copy of taps (read at launch)
   int nogate;               // peaks whatever sigma0 (DEBUG_ALWAYS_FIND_PEAKS)
 };
-// Shared memory of the FIR launch.
-size_t fir_smem_bytes(const SmoothArgs &a);
 cudaError_t smooth_planes(const SmoothArgs &a, cudaStream_t s);
 // scale = 1: per-width mean/std (normalisation); 0: planes left as they
 // are.  A launch holding width 0 then forms the beams' gate statistics.

@@ -129,7 +129,7 @@ struct hella_ctx {
   float *h_cand_v = nullptr;
   int *h_total = nullptr;
   std::vector<hella_cand> peaks;
-  std::vector<int> tap_n;
+  std::vector<float> taps;  // host copy of d_taps
   bool loaded = false, flagged = false, smoothed = false;
   int dd_beam = -1;
   int *d_err = nullptr;  // device status word of the staging waits
@@ -188,6 +188,7 @@ hg::SmoothArgs smooth_args(hella_ctx *c) {
   a.taps = c->d_taps;
   a.tap_off = c->d_tapoff;
   a.tap_n = c->d_tapn;
+  a.taps_host = c->taps.data();
   a.snr = c->p.snr;
   a.nogate = c->p.always_find_peaks != 0;
   return a;
@@ -461,7 +462,7 @@ hella_status hella_create(hella_ctx **out, const hella_params *p) {
   std::vector<float> taps;
   std::vector<int> off, n;
   hg::smoothing_taps(*p, c->nbox, &taps, &off, &n);
-  c->tap_n = n;
+  c->taps = taps;
   if ((s = dalloc(c, (void **)&c->d_taps, taps.size() * 4)) != HELLA_OK) return fail(s);
   if ((s = dalloc(c, (void **)&c->d_tapoff, off.size() * 4)) != HELLA_OK) return fail(s);
   if ((s = dalloc(c, (void **)&c->d_tapn, n.size() * 4)) != HELLA_OK) return fail(s);

@@ -16,16 +16,13 @@
 // i.e. the DM weights factored out of the 2-D kernel, whose middle row
 // supplies the time taps.  Borders replicate (NPP_BORDER_REPLICATE).
 //
-// Kernels.  The FIR stages a row's y values chunk by chunk in shared memory
-// in a 16-phase layout, so that each thread keeps a sliding window of 16
-// outputs in registers and reads one shared word per tap for all 16; every
-// width is produced from the same staged chunk, and the row-mean partials
-// of the reference's order (thread j sums columns j, j+256, ...) are
-// accumulated as the chunk is written, so the plane is written once and
-// read once more for the variance.  k_firR (spans up to 2048 samples) does
-// this with constant-offset window loads and two width groups per row;
-// k_fir, with runtime window addresses, takes wider spans.  Row maxima let
-// the peak pass skip rows that cannot hold a candidate.
+// Kernels.  k_firS filters a row with every width up to 32 from a register
+// window (a block per row), k_firL with one larger width and a sliding window
+// (a block per row and width).  Both form the
+// row-mean partials of the reference's order (thread j sums columns j, j+256,
+// ...) as they go; the plane is written once and read once more for the
+// variance.  Row maxima let the peak pass skip rows that cannot hold
+// a candidate.
 #include "hg_internal.h"
 
 #include <algorithm>
@@ -33,9 +30,7 @@
 namespace hg {
 namespace {
 
-constexpr int kR = 16;            // outputs per thread (taps padded to kR)
-constexpr int kT = 256;           // threads per row block
-constexpr int kCH = kR * kT;      // outputs per chunk
+constexpr int kT = 256;  // threads per row block of the statistics passes
 
 __device__ __forceinline__ float block256_tree(const float *p) {
   // p: 256 partials in shared memory; called by one whole warp, returns in
@@ -63,460 +58,379 @@ __device__ __forceinline__ const SmoothBeam &row_beam(const SmoothArgs &a, int g
   return B;
 }
 
-// One block per (beam, row): widths w0..w0+nw-1 of the row from one staged
-// chunk of y values.  taps of those widths are copied to shared memory.
-__global__ void __launch_bounds__(kT) k_fir(SmoothArgs a) {
-  extern __shared__ __align__(16) float sm[];
-  int r;
-  const SmoothBeam &B = row_beam(a, blockIdx.x, &r);
-  if (!*B.active) return;
-  const int w0 = a.w0, nw = a.nw, h = B.h, tid = threadIdx.x;
-  const int span = 2 * (a.wmin << (w0 + nw - 1));
-  const int ylen = kCH + span + 2 * kR;
-  const int M = (ylen + kR - 1) / kR;
-  const int tap0 = a.tap_off[w0];
-  int ntaps_total = 0;
-  for (int b = w0; b < w0 + nw; ++b) ntaps_total += a.tap_n[b];
-  float *taps = sm;
-  float *Y = taps + ((ntaps_total + 3) / 4) * 4;
-  float *out_s = Y + kR * M;
-  float *part_s = out_s + kCH;
-  float *max_s = part_s + nw * kT;
-  for (int i = tid; i < ntaps_total; i += kT) taps[i] = a.taps[tap0 + i];
-  for (int j = 0; j < nw; ++j) {
-    part_s[j * kT + tid] = 0.f;
-    max_s[j * kT + tid] = -INFINITY;
-  }
-  const float *ra = B.dd + (size_t)r * B.dd_stride;
-  const float *rb = ra + B.dd_stride;
-  const float *rc = rb + B.dd_stride;
-  const int nwcol = 256 * (a.ntime_out / 256);
-  const int org = a.wmax / 2 - (a.anchor ? span : 0);
+// 32 bytes to global memory in one store (a whole sector a lane).
+__device__ __forceinline__ void store8(float *p, const float *v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
 
-  for (int cs = 0; cs < a.ntime_out; cs += kCH) {
-    __syncthreads();
-    for (int x = tid; x < kR * M; x += kT) {
-      int col = cs + org + x;
-      col = col < 0 ? 0 : (col >= a.ntime_dd ? a.ntime_dd - 1 : col);
-      Y[(x % kR) * M + x / kR] = __fmaf_rn(0.3f, __fadd_rn(ra[col], rc[col]), rb[col]);
-    }
-    __syncthreads();
-    for (int j = 0; j < nw; ++j) {
-      const int b = w0 + j;
-      const int smw = a.wmin << b;
-      const int off = a.anchor ? span - 2 * smw : 0;
-      const float *tp = taps + a.tap_off[b] - tap0;
-      const int ntap = 2 * smw + 1, nblk = ntap / kR, tail = ntap - nblk * kR;
-      const int base = kR * tid + off;
-      // win[] slides over y; pre[kk] is where the slot refilled at tap kk of
-      // the first block of kR taps lives in Y (later blocks add one column)
-      float acc[kR], win[kR];
-      int pre[kR];
-#pragma unroll
-      for (int i = 0; i < kR; ++i) {
-        acc[i] = 0.f;
-        const int x = base + i, xr = base + i + kR;
-        win[i] = Y[(x % kR) * M + x / kR];
-        pre[i] = (xr % kR) * M + xr / kR;
-      }
-      int kq = 0;
-      for (; kq < nblk; ++kq) {
-#pragma unroll
-        for (int k4 = 0; k4 < kR; k4 += 4) {
-          const float4 c4 = *reinterpret_cast<const float4 *>(tp + kq * kR + k4);
-          const float cfs[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const int kk = k4 + jj;
-#pragma unroll
-            for (int i = 0; i < kR; ++i) acc[i] = __fmaf_rn(cfs[jj], win[(i + kk) % kR], acc[i]);
-            win[kk] = Y[pre[kk] + kq];
-          }
-        }
-      }
-      // the last partial block: the same steps, stopping after `tail` taps
-      // (no zero taps are issued; every width of 17 taps or more has a
-      // 1-tap tail)
-      if (tail) {
-#pragma unroll
-        for (int k4 = 0; k4 < kR; k4 += 4) {
-          if (k4 >= tail) break;
-          const float4 c4 = *reinterpret_cast<const float4 *>(tp + kq * kR + k4);
-          const float cfs[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const int kk = k4 + jj;
-            if (kk >= tail) break;
-#pragma unroll
-            for (int i = 0; i < kR; ++i) acc[i] = __fmaf_rn(cfs[jj], win[(i + kk) % kR], acc[i]);
-            win[kk] = Y[pre[kk] + kq];
-          }
-        }
-      }
-      float4 *o4 = reinterpret_cast<float4 *>(out_s + kR * tid);
-#pragma unroll
-      for (int i = 0; i < kR / 4; ++i) o4[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
-      __syncthreads();
-      float *dst = B.boxes + ((size_t)j * h + r) * a.ntime_out;
-      float ps = part_s[j * kT + tid], mx = max_s[j * kT + tid];
-#pragma unroll
-      for (int m = 0; m < kR; ++m) {
-        const int jc = tid + kT * m, col = cs + jc;
-        if (col < a.ntime_out) {
-          const float v = out_s[jc];
-          dst[col] = v;
-          mx = fmaxf(mx, v);
-          if (col < nwcol) ps = __fadd_rn(ps, v);
-        }
-      }
-      part_s[j * kT + tid] = ps;
-      max_s[j * kT + tid] = mx;
-      __syncthreads();
-    }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// The three dedispersed rows a smoothed row is made of, and its y values.
+struct YRows {
+  const float *a, *b, *c;
+  int n;       // columns
+  bool vec;    // 16-byte loads of columns 4k are aligned
+  __device__ __forceinline__ YRows(const SmoothBeam &B, int r, int ntime_dd)
+      : a(B.dd + (size_t)r * B.dd_stride), b(a + B.dd_stride), c(b + B.dd_stride), n(ntime_dd),
+        vec((reinterpret_cast<uintptr_t>(B.dd) & 15) == 0 && B.dd_stride % 4 == 0) {}
+  static __device__ __forceinline__ float y(float a, float b, float c) { return __fmaf_rn(0.3f, __fadd_rn(a, c), b); }
+  __device__ __forceinline__ float at(int col) const {  // borders replicate
+    col = col < 0 ? 0 : (col >= n ? n - 1 : col);
+    return y(a[col], b[col], c[col]);
   }
-  __syncthreads();
-  for (int j = tid >> 5; j < nw; j += kT / 32) {
-    const float tot = block256_tree(part_s + j * kT);
-    float mx = -INFINITY;
-    for (int i = threadIdx.x & 31; i < kT; i += 32) mx = fmaxf(mx, max_s[j * kT + i]);
-    for (int off = 16; off > 0; off /= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    if ((tid & 31) == 0) {
-      B.rowmean[(size_t)(w0 + j) * h + r] = __fdiv_rn(tot, (float)nwcol);
-      B.rowmax[(size_t)(w0 + j) * h + r] = mx;
-    }
+};
+
+// Row total of 256 partials p and maximum mx (every lane's), by one warp.
+__device__ __forceinline__ void row_finish(const SmoothBeam &B, int b, int r, const float *p, float mx, int nwcol) {
+  const float tot = block256_tree(p);
+  for (int o = 16; o > 0; o /= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) {
+    B.rowmean[(size_t)b * B.h + r] = __fdiv_rn(tot, (float)nwcol);
+    B.rowmax[(size_t)b * B.h + r] = mx;
   }
 }
 
-// k_firR: the arithmetic of k_fir with R outputs per thread (R = 16 or
-// 32) and 128 threads per (row, width group); widths [w0, split) form
-// group 0 and [split, w0 + nw) group 1 (blockIdx.y), so that a short list
-// of long rows still fills the GPU.  The chunk's y values are staged in an
-// R-phase layout with a compile-time phase stride M and 2R phase rows,
-//   Y[p * M + c] = y(R c + p)   (p < 2R, c < M),
-// so that for every width (off = R O + o) window element n of thread t is
-// Y[(o + n % R) * M + t + O + n / R]: one base address per width, and
-// every load of the tap loop sits at a constant offset from it.  Outputs
-// go to global memory straight from registers; the row-mean partials of
-// the reference's order (owner j sums columns j, j + 256, ...) read them
-// back through a swizzled shared transpose (conflict-free both ways).
-constexpr int kTF = 128;  // threads per block
+// k_firS: the widths 1, 2, 4 .. 32 (wmin 1) of a launch, a block of four warps
+// per row.  An iteration makes 1024 outputs of every width, a warp 256 of
+// them, lane t outputs 8t .. 8t + 7 from the 72 y values they read, kept in
+// registers, so that a tap is eight multiply-adds on registers and a constant:
+// the taps are kernel arguments.  The y values sit in shared memory as groups
+// of 8 at a pitch of 12 words (conflict-free 16-byte reads at a lane stride of
+// one group), in two buffers: the 64 values two iterations share are copied to
+// the front of the other one.  The three rows are copied an iteration ahead
+// (cp.async, each thread the columns it reads back; in 4-byte pieces at the
+// row's ends and where rows are not 16-byte aligned).  The outputs also go to
+// shared memory, where thread i keeps the row-mean partials of columns 4i ..
+// 4i + 3 (mod 256) of half of the widths and adds the warps' chunks in order:
+// two block barriers an iteration.  Bound by issue (about 1330 instructions for
+// a warp's 256 outputs, 1056 of them multiply-adds, issued 70 % of the cycles).
+// 8923 rows x 32768 x 6 widths: 1.92 ms, with rows staged by plain loads, taps
+// in shared memory and a barrier-separated transpose of 2048 outputs 3.1 ms;
+// 493 rows x 16384: 85 us against 103.  Three blocks an SM (132 registers)
+// rather than four (124): 1.92 against 2.05 ms; a warp a row with the partials
+// in registers 1.81 ms, but 105 us on the 493 rows, one warp's walk being long.
+constexpr int kSO = 8;                   // outputs per lane
+constexpr int kSWarps = 4;               // warps per block
+constexpr int kST = 32 * kSWarps;        // threads per block
+constexpr int kSC = kST * kSO;           // outputs per iteration
+constexpr int kSSpan = 64;               // span of width 32
+constexpr int kSW = 6;                   // widths 1, 2, 4, 8, 16, 32
+constexpr int kSWin = kSO + kSSpan;      // y values a lane reads (72)
+constexpr int kSPitch = 12;              // words from one group of 8 to the next
+constexpr int kSY = (kSC + kSSpan) / 8 * kSPitch;
+constexpr int kSRaw = 3 * kSC;           // words of an iteration's staged rows
+constexpr size_t kSSmem = sizeof(float) * (2 * kSY + kSRaw + kSW * kSC);
+__host__ __device__ constexpr int small_tap(int b) { return 2 * ((1 << b) - 1) + b; }  // first tap of width 2^b
+struct SmallTaps {
+  float t[small_tap(kSW)];
+};
+// Word of 16-byte slot s: the two slots of a lane's 8 values trade places in every other eight, so
+// that lanes reading or writing slots 2t (or 2t + 1) meet no bank conflict.
+__device__ __forceinline__ int slot_word(int s) { return 4 * (s ^ ((s >> 3) & 1)); }
 
-// float4 slot q of thread t's R outputs sits at slot q ^ fir_swz_key(t).
-template <int R>
-__device__ __forceinline__ int fir_swz_key(int t) {
-  return R == 32 ? (t & 7) : ((t >> 1) & 3);
-}
-// Transposed position of chunk column c.
-template <int R>
-__device__ __forceinline__ int fir_swz(int c) {
-  const int t = c / R, q = (c % R) >> 2;
-  return R * t + 4 * (q ^ fir_swz_key<R>(t)) + (c & 3);
-}
-
-template <int R, int M>
-__global__ void __launch_bounds__(kTF, R == 32 ? 3 : 5) k_firR(SmoothArgs a) {
-  constexpr int kC = R * kTF;  // outputs per chunk
-  extern __shared__ __align__(16) float sm[];
-  int r;
-  const SmoothBeam &B = row_beam(a, blockIdx.x, &r);
-  if (!*B.active) return;
-  const int wb = blockIdx.y == 0 ? a.w0 : a.split, we = blockIdx.y == 0 ? a.split : a.w0 + a.nw;
-  const int nw = we - wb;
-  if (nw <= 0) return;
-  const int h = B.h, tid = threadIdx.x;
-  const int span = 2 * (a.wmin << (a.w0 + a.nw - 1));
-  const int tap0 = a.tap_off[wb];
-  int ntaps_total = 0;
-  for (int b = wb; b < we; ++b) ntaps_total += a.tap_n[b];
-  float *taps = sm;
-  float *Y = taps + ((ntaps_total + 3) / 4) * 4;
-  float *out_s = Y + 2 * R * M;
-  float *part_s = out_s + kC;        // [nw][256] row-mean partials
-  float *max_s = part_s + nw * 256;  // [nw][kTF] row maxima
-  for (int i = tid; i < ntaps_total; i += kTF) taps[i] = a.taps[tap0 + i];
-  for (int j = 0; j < nw; ++j) {
-    part_s[j * 256 + tid] = 0.f;
-    part_s[j * 256 + kTF + tid] = 0.f;
-    max_s[j * kTF + tid] = -INFINITY;
-  }
-  const float *ra = B.dd + (size_t)r * B.dd_stride;
-  const float *rb = ra + B.dd_stride;
-  const float *rc = rb + B.dd_stride;
-  const int nwcol = 256 * (a.ntime_out / 256);
-  const int org = a.wmax / 2 - (a.anchor ? span : 0);
-
-  constexpr int NY = R * (M + 1);                // staged y values
-  constexpr int NX = (NY + kTF - 1) / kTF;       // per thread
-  constexpr int XB = 6;                          // loads in flight per thread
-  for (int cs = 0; cs < a.ntime_out; cs += kC) {
-    __syncthreads();
-    for (int i0 = 0; i0 < NX; i0 += XB) {
-      float va[XB], vb[XB], vc[XB];
-#pragma unroll
-      for (int u = 0; u < XB; ++u) {
-        int col = cs + org + tid + (i0 + u) * kTF;
-        col = col < 0 ? 0 : (col >= a.ntime_dd ? a.ntime_dd - 1 : col);
-        va[u] = ra[col];
-        vb[u] = rb[col];
-        vc[u] = rc[col];
-      }
-#pragma unroll
-      for (int u = 0; u < XB; ++u) {
-        const int x = tid + (i0 + u) * kTF;
-        const int c = x / R, p = x % R;
-        if (x < NY) {
-          const float y = __fmaf_rn(0.3f, __fadd_rn(va[u], vc[u]), vb[u]);
-          if (c < M) Y[p * M + c] = y;
-          if (c >= 1) Y[(p + R) * M + c - 1] = y;
-        }
-      }
-    }
-    __syncthreads();
-    const bool valid = cs + R * tid < a.ntime_out;  // ntime_out % R == 0
-    for (int j = 0; j < nw; ++j) {
-      const int b = wb + j;
-      const int smw = a.wmin << b;
-      const int off = a.anchor ? span - 2 * smw : 0;
-      const float *tp = taps + a.tap_off[b] - tap0;
-      const int ntap = 2 * smw + 1, nblk = ntap / R, tail = ntap % R;
-      const float *Yp = Y + (off % R) * M + tid + off / R;
-      // win[(i + kk) % R] holds y at window element R kq + kk + i of output
-      // i; slot kk is refilled after step kk of block kq
-      float acc[R], win[R];
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        acc[i] = 0.f;
-        win[i] = Yp[i * M];
-      }
-      // taps are read one group of four ahead (cn); ntap is odd, so the
-      // group after the last full block is the tail's first
-      float4 cn = *reinterpret_cast<const float4 *>(tp);
-      int kq = 0;
-      for (; kq < nblk; ++kq) {
-        const float *Yq = Yp + kq + 1;
-        const float *tq = tp + kq * R;
-#pragma unroll
-        for (int k4 = 0; k4 < R; k4 += 4) {
-          const float4 c4 = cn;
-          cn = *reinterpret_cast<const float4 *>(tq + k4 + 4);
-          const float cfs[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const int kk = k4 + jj;
-#pragma unroll
-            for (int i = 0; i < R; ++i) acc[i] = __fmaf_rn(cfs[jj], win[(i + kk) % R], acc[i]);
-            win[kk] = Yq[kk * M];
-          }
-        }
-      }
-      if (tail) {  // the last `tail` taps (no zero taps are issued)
-        const float *Yq = Yp + kq + 1;
-        const float *tq = tp + kq * R;
-#pragma unroll
-        for (int k4 = 0; k4 < R; k4 += 4) {
-          if (k4 >= tail) break;
-          const float4 c4 = cn;
-          if (k4 + 4 < tail) cn = *reinterpret_cast<const float4 *>(tq + k4 + 4);
-          const float cfs[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const int kk = k4 + jj;
-            if (kk >= tail) break;
-#pragma unroll
-            for (int i = 0; i < R; ++i) acc[i] = __fmaf_rn(cfs[jj], win[(i + kk) % R], acc[i]);
-            win[kk] = Yq[kk * M];
-          }
-        }
-      }
-      if (valid) {
-        float4 *dst = reinterpret_cast<float4 *>(B.boxes + ((size_t)(b - a.w0) * h + r) * a.ntime_out + cs +
-                                                 R * tid);
-        float mx = max_s[j * kTF + tid];
-#pragma unroll
-        for (int q = 0; q < R / 4; ++q) {
-          dst[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-          mx = fmaxf(fmaxf(fmaxf(mx, acc[4 * q]), fmaxf(acc[4 * q + 1], acc[4 * q + 2])), acc[4 * q + 3]);
-        }
-        max_s[j * kTF + tid] = mx;
-      }
-      const int key = fir_swz_key<R>(tid);
-#pragma unroll
-      for (int q = 0; q < R / 4; ++q)
-        *reinterpret_cast<float4 *>(out_s + R * tid + 4 * (q ^ key)) =
-            make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-      __syncthreads();
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int jo = tid + kTF * hh, c0 = cs + jo;
-        const int nm = c0 < nwcol ? min(kC / 256, (nwcol - c0 + 255) >> 8) : 0;
-        const float *src = out_s + fir_swz<R>(jo);  // column jo + 256 m at src[256 m]
-        float ps = part_s[j * 256 + jo];
-#pragma unroll
-        for (int m = 0; m < kC / 256; ++m)
-          if (m < nm) ps = __fadd_rn(ps, src[256 * m]);
-        part_s[j * 256 + jo] = ps;
-      }
-      __syncthreads();
-    }
-  }
-  for (int j = tid >> 5; j < nw; j += kTF / 32) {
-    const float tot = block256_tree(part_s + j * 256);
-    float mx = -INFINITY;
-    for (int i = threadIdx.x & 31; i < kTF; i += 32) mx = fmaxf(mx, max_s[j * kTF + i]);
-    for (int o = 16; o > 0; o /= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0) {
-      B.rowmean[(size_t)(wb + j) * h + r] = __fdiv_rn(tot, (float)nwcol);
-      B.rowmax[(size_t)(wb + j) * h + r] = mx;
-    }
-  }
-}
-
-// k_firS: the arithmetic of k_firR for launches whose widths are all at
-// most 32 (wmin 1, wmax <= 64: spans of at most 64 samples), the widths of
-// the plain, batched and streaming configurations, whose few taps per width
-// left k_firR's per-width window set-up, stores, transposes and barriers as
-// large as the multiply-adds.  256 threads, 8 outputs each (the same
-// 2048-output chunks); thread t keeps the 72 y values its outputs read in
-// registers, so every tap is eight multiply-adds on registers; each width's
-// outputs get their own slot of a shared buffer, so one barrier pair per
-// chunk serves the row-mean partials of every width.  Per output: the same
-// multiply-add chain over the taps in order from zero, the same y values
-// and the same partial order as k_firR.
-constexpr int kSO = 8;                  // outputs per thread
-constexpr int kST = 256;                // threads per block
-constexpr int kSC = kSO * kST;          // outputs per chunk (k_firR's)
-constexpr int kSSpan = 64;              // largest span served
-constexpr int kSW = 6;                  // widths 1, 2, 4, 8, 16, 32
-constexpr int kSWin = kSO + kSSpan;     // y values a thread reads (72)
-constexpr int kSY = kSC + kSSpan + kSO; // y values staged per chunk (2120)
-constexpr int kSTap = 68;               // taps kept per width (65 used at most, float4 loads)
-static_assert(kSWin % 4 == 0 && kSY % 4 == 0 && kSTap % 4 == 0, "float4 staging");
-
-// One width (2 SM + 1 taps) of a thread's 8 outputs from its register window.
+// One width (2 SM + 1 taps) of a lane's 8 outputs from its register window.
 template <int SM, int ANCHOR>
 __device__ __forceinline__ void firS_width(const float (&win)[kSWin], const float *tp, float (&acc)[kSO]) {
   constexpr int NT = 2 * SM + 1, OFF = ANCHOR ? kSSpan - 2 * SM : 0;
 #pragma unroll
   for (int i = 0; i < kSO; ++i) acc[i] = 0.f;
 #pragma unroll
-  for (int n4 = 0; n4 < NT; n4 += 4) {
-    const float4 c4 = *reinterpret_cast<const float4 *>(tp + n4);
-    const float cf[4] = {c4.x, c4.y, c4.z, c4.w};
+  for (int n = 0; n < NT; ++n)
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const int n = n4 + jj;
-      if (n < NT) {
-#pragma unroll
-        for (int i = 0; i < kSO; ++i) acc[i] = __fmaf_rn(cf[jj], win[OFF + i + n], acc[i]);
-      }
-    }
-  }
+    for (int i = 0; i < kSO; ++i) acc[i] = __fmaf_rn(tp[n], win[OFF + i + n], acc[i]);
 }
 
 template <int ANCHOR>
-__global__ void __launch_bounds__(kST, 2) k_firS(SmoothArgs a) {
+__global__ void __launch_bounds__(kST, 3) k_firS(SmoothArgs a, const __grid_constant__ SmallTaps taps, int b0, int b1) {
   extern __shared__ __align__(16) float sm[];
-  float *Ys = sm;                     // [kSY]
-  float *out_s = Ys + kSY;            // [kSW][kSC]
-  float *part_s = out_s + kSW * kSC;  // [kSW][256]
-  float *taps = part_s + kSW * 256;   // [kSW][kSTap]
   int r;
   const SmoothBeam &B = row_beam(a, blockIdx.x, &r);
   if (!*B.active) return;
-  const int h = B.h, tid = threadIdx.x, bw0 = a.w0, bw1 = a.w0 + a.nw;
-  for (int i = tid; i < kSW * kSTap; i += kST) {
-    const int b = i / kSTap, n = i - b * kSTap;
-    taps[i] = b < a.nbox && n < a.tap_n[b] ? a.taps[a.tap_off[b] + n] : 0.f;
-  }
-  for (int i = tid; i < kSW * 256; i += kST) part_s[i] = 0.f;
-  float mx[kSW];
+  float *Y = sm, *const raw = sm + 2 * kSY, *const out_s = raw + kSRaw;  // Y: two buffers, this iteration's
+  const int tid = threadIdx.x, warp = tid >> 5, nout = a.ntime_out;
+  const YRows rows(B, r, a.ntime_dd);
+  const int org = a.wmax / 2 - (ANCHOR ? kSSpan : 0);
+  const bool vec = rows.vec && org % 4 == 0;
+  float mx[kSW], part[kSW / 2][4];
 #pragma unroll
   for (int b = 0; b < kSW; ++b) mx[b] = -INFINITY;
-  const float *ra = B.dd + (size_t)r * B.dd_stride;
-  const float *rb = ra + B.dd_stride;
-  const float *rc = rb + B.dd_stride;
-  const int nwcol = 256 * (a.ntime_out / 256);
-  const int org = a.wmax / 2 - (ANCHOR ? kSSpan : 0);
-  constexpr int NL = (kSY + kST - 1) / kST;  // staged values per thread
-  for (int cs = 0; cs < a.ntime_out; cs += kSC) {
-    __syncthreads();  // the previous chunk's shared reads are done
-    {
-      float va[NL], vb[NL], vc[NL];
 #pragma unroll
-      for (int u = 0; u < NL; ++u) {
-        const int sx = tid + u * kST;
-        int col = cs + org + sx;
-        col = col < 0 ? 0 : (col >= a.ntime_dd ? a.ntime_dd - 1 : col);
-        if (sx < kSY) {
-          va[u] = ra[col];
-          vb[u] = rb[col];
-          vc[u] = rc[col];
+  for (int b = 0; b < kSW / 2; ++b)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) part[b][i] = 0.f;
+  const uint32_t raw0 = (uint32_t)__cvta_generic_to_shared(raw);
+  const int sl0 = slot_word(2 * tid), sl1 = slot_word(2 * tid + 1);
+  auto load = [&](int cs) {  // this thread's 8 columns of the rows that enter with the outputs from cs
+    if (cs < nout) {
+      const int w0 = cs + org + kSSpan, c0 = w0 + kSO * tid;
+      const float *src[3] = {rows.a, rows.b, rows.c};
+      if (vec && w0 >= 0 && w0 + kSC <= rows.n) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          cp_async16(raw0 + 4u * (k * kSC + sl0), src[k] + c0);
+          cp_async16(raw0 + 4u * (k * kSC + sl1), src[k] + c0 + 4);
+        }
+      } else {
+        for (int i = 0; i < kSO; ++i) {
+          const int col = min(max(c0 + i, 0), rows.n - 1), w = (i < 4 ? sl0 : sl1) + (i & 3);
+          for (int k = 0; k < 3; ++k) cp_async4(raw0 + 4u * (k * kSC + w), src[k] + col);
         }
       }
-#pragma unroll
-      for (int u = 0; u < NL; ++u) {
-        const int sx = tid + u * kST;
-        if (sx < kSY) Ys[sx] = __fmaf_rn(0.3f, __fadd_rn(va[u], vc[u]), vb[u]);
-      }
     }
+    cp_async_commit();
+  };
+  load(0);
+  if (tid < kSSpan) Y[kSPitch * (tid / 8) + tid % 8] = rows.at(org + tid);
+  const int pb = 3 * (tid >> 6), pq = tid & 63;  // partials: widths pb .. pb + 2, slot pq of each chunk
+#pragma unroll 1
+  for (int cs = 0, buf = 0; cs < nout; cs += kSC, buf ^= 1) {
+    Y = sm + buf * kSY;
+    cp_async_wait<0>();  // the rows this thread copied
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float *x = raw + (h ? sl1 : sl0);
+      const float4 u = *reinterpret_cast<const float4 *>(x), v = *reinterpret_cast<const float4 *>(x + kSC),
+                   w = *reinterpret_cast<const float4 *>(x + 2 * kSC);
+      *reinterpret_cast<float4 *>(Y + kSPitch * (kSSpan / 8 + tid) + 4 * h) =
+          make_float4(YRows::y(u.x, v.x, w.x), YRows::y(u.y, v.y, w.y), YRows::y(u.z, v.z, w.z),
+                      YRows::y(u.w, v.w, w.w));
+    }
+    load(cs + kSC);
     __syncthreads();
     float win[kSWin];
 #pragma unroll
     for (int q = 0; q < kSWin / 4; ++q) {
-      const float4 v = *reinterpret_cast<const float4 *>(Ys + kSO * tid + 4 * q);
+      const float4 v = *reinterpret_cast<const float4 *>(Y + kSPitch * (tid + q / 2) + 4 * (q & 1));
       win[4 * q] = v.x;
       win[4 * q + 1] = v.y;
       win[4 * q + 2] = v.z;
       win[4 * q + 3] = v.w;
     }
-    const bool valid = cs + kSO * tid < a.ntime_out;  // ntime_out % kSO == 0
+    if (tid < kSSpan / 4) {  // the next iteration's first 64 values
+      const int o = kSPitch * (tid / 2) + 4 * (tid & 1);
+      *reinterpret_cast<float4 *>(sm + (buf ^ 1) * kSY + o) = *reinterpret_cast<const float4 *>(Y + o + kSPitch * (kSC / 8));
+    }
+    const bool valid = cs + kSO * tid < nout;  // nout % 8 == 0
     float acc[kSO];
     auto emit = [&](int b) {
       if (valid) {
-        float4 *dst = reinterpret_cast<float4 *>(B.boxes + ((size_t)(b - a.w0) * h + r) * a.ntime_out + cs +
-                                                 kSO * tid);
-        dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        store8(B.boxes + ((size_t)(b - a.w0) * B.h + r) * nout + cs + kSO * tid, acc);
 #pragma unroll
-        for (int i = 0; i < kSO; ++i) mx[b] = fmaxf(mx[b], acc[i]);
+        for (int i = 0; i < kSO; i += 2) mx[b] = max3(mx[b], acc[i], acc[i + 1]);
       }
-      float4 *o = reinterpret_cast<float4 *>(out_s + b * kSC + kSO * tid);
-      o[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-      o[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+      *reinterpret_cast<float4 *>(out_s + b * kSC + sl0) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      *reinterpret_cast<float4 *>(out_s + b * kSC + sl1) = make_float4(acc[4], acc[5], acc[6], acc[7]);
     };
-    if (bw0 <= 0 && 0 < bw1) { firS_width<1, ANCHOR>(win, taps + 0 * kSTap, acc); emit(0); }
-    if (bw0 <= 1 && 1 < bw1) { firS_width<2, ANCHOR>(win, taps + 1 * kSTap, acc); emit(1); }
-    if (bw0 <= 2 && 2 < bw1) { firS_width<4, ANCHOR>(win, taps + 2 * kSTap, acc); emit(2); }
-    if (bw0 <= 3 && 3 < bw1) { firS_width<8, ANCHOR>(win, taps + 3 * kSTap, acc); emit(3); }
-    if (bw0 <= 4 && 4 < bw1) { firS_width<16, ANCHOR>(win, taps + 4 * kSTap, acc); emit(4); }
-    if (bw0 <= 5 && 5 < bw1) { firS_width<32, ANCHOR>(win, taps + 5 * kSTap, acc); emit(5); }
+    if (b0 <= 5 && 5 < b1) { firS_width<32, ANCHOR>(win, taps.t + small_tap(5), acc); emit(5); }
+    if (b0 <= 4 && 4 < b1) { firS_width<16, ANCHOR>(win, taps.t + small_tap(4), acc); emit(4); }
+    if (b0 <= 3 && 3 < b1) { firS_width<8, ANCHOR>(win, taps.t + small_tap(3), acc); emit(3); }
+    if (b0 <= 2 && 2 < b1) { firS_width<4, ANCHOR>(win, taps.t + small_tap(2), acc); emit(2); }
+    if (b0 <= 1 && 1 < b1) { firS_width<2, ANCHOR>(win, taps.t + small_tap(1), acc); emit(1); }
+    if (b0 <= 0 && 0 < b1) { firS_width<1, ANCHOR>(win, taps.t + small_tap(0), acc); emit(0); }
     __syncthreads();
-    // row-mean partials in the reference's order: owner jo adds columns jo, jo + 256, ...
-    const int c0 = cs + tid;
-    const int nm = c0 < nwcol ? min(kSC / 256, (nwcol - c0 + 255) >> 8) : 0;
-    for (int b = bw0; b < bw1; ++b) {
-      float ps = part_s[b * 256 + tid];
+    const int nm = min(kSWarps, (nout - cs) / 256);  // whole chunks: their columns count for the row mean
 #pragma unroll
-      for (int m = 0; m < kSC / 256; ++m)
-        if (m < nm) ps = __fadd_rn(ps, out_s[b * kSC + tid + 256 * m]);
-      part_s[b * 256 + tid] = ps;
-    }
+    for (int j = 0; j < kSW / 2; ++j)
+      if (b0 <= pb + j && pb + j < b1) {
+#pragma unroll
+        for (int m = 0; m < kSWarps; ++m)
+          if (m < nm) {
+            const float4 v = *reinterpret_cast<const float4 *>(out_s + (pb + j) * kSC + slot_word(64 * m + pq));
+            part[j][0] = __fadd_rn(part[j][0], v.x);
+            part[j][1] = __fadd_rn(part[j][1], v.y);
+            part[j][2] = __fadd_rn(part[j][2], v.z);
+            part[j][3] = __fadd_rn(part[j][3], v.w);
+          }
+      }
   }
+  // row totals: partials and the warps' maxima through shared memory, a warp a width
   __syncthreads();
 #pragma unroll
-  for (int b = 0; b < kSW; ++b)
-    if (b >= bw0 && b < bw1) out_s[b * 256 + tid] = mx[b];
+  for (int j = 0; j < kSW / 2; ++j)
+    *reinterpret_cast<float4 *>(out_s + (pb + j) * 256 + 4 * pq) =
+        make_float4(part[j][0], part[j][1], part[j][2], part[j][3]);
+#pragma unroll
+  for (int b = 0; b < kSW; ++b) sm[b * kST + tid] = mx[b];
   __syncthreads();
-  for (int b = bw0 + (tid >> 5); b < bw1; b += kST / 32) {
-    const float tot = block256_tree(part_s + b * 256);
+  const int nwcol = 256 * (nout / 256);
+  for (int b = b0 + warp; b < b1; b += kSWarps) {
     float m = -INFINITY;
-    for (int i = threadIdx.x & 31; i < kST; i += 32) m = fmaxf(m, out_s[b * 256 + i]);
-    for (int o = 16; o > 0; o /= 2) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((tid & 31) == 0) {
-      B.rowmean[(size_t)b * h + r] = __fdiv_rn(tot, (float)nwcol);
-      B.rowmax[(size_t)b * h + r] = m;
+#pragma unroll
+    for (int i = 0; i < kSWarps; ++i) m = fmaxf(m, sm[b * kST + 32 * i + (tid & 31)]);
+    row_finish(B, b, r, out_s + b * 256, m, nwcol);
+  }
+}
+
+// k_firL: one width of any size, a block of four warps per (row, width), the
+// widest width's blocks first so that the short ones fill the last wave.  An
+// iteration makes 2048 outputs, thread t outputs 16t .. 16t + 15 with a
+// sliding window of 16 y values in registers: four taps are 64 multiply-adds,
+// one 16-byte read of the y values that enter the window and one of the taps
+// (both a group of four ahead).  The iteration's y values and the span before
+// them sit in shared memory as rows of 16 at a pitch of 20 words: window
+// element n of thread t is word 20 (t + n / 16) + n % 16, a constant offset
+// from one base, conflict-free at a lane stride of one row.  The outputs also
+// go to shared memory (16-byte slots permuted, conflict-free), where thread i
+// adds those of columns 2i and 2i + 1 (mod 256) to its row-mean partials in
+// order; three block barriers an iteration.  Bound by multiply-add issue: 79 %
+// of the cycles issue, the rest are mostly dispatch stalls of warps that are
+// ready.  2499 rows x 65536 x widths 64, 128, 256: 5.09 ms = 1.47e11 multiply-
+// adds at 72 % of the FP32 rate (with width 1-32's k_firS 6.14 ms; one kernel
+// for all nine widths with a barrier pair per width and 2048 outputs 7.50 ms).
+// A warp a row walks too long where rows are few: 394 rows x 10016, 190 us
+// against 143.  Six blocks an SM (85 registers) 5.09 ms, five 5.17.
+constexpr int kLO = 16;          // outputs per thread
+constexpr int kLT = 128;         // threads per block
+constexpr int kLC = kLT * kLO;   // outputs per iteration
+constexpr int kLPitch = 20;      // words from one row of 16 y values to the next
+__host__ __device__ constexpr int firL_taps(int smw) { return (2 * smw + 1 + 15) / 16 * 16 + 8; }
+// rows of 16: the threads', the taps' blocks, one block read ahead
+__host__ __device__ constexpr int firL_rows(int smw) { return kLT + 2 + (2 * smw + 1) / 16; }
+
+__device__ __forceinline__ int firL_word(int x) { return kLPitch * (x / 16) + x % 16; }
+
+__global__ void __launch_bounds__(kLT, 6) k_firL(SmoothArgs a, int bend) {
+  extern __shared__ __align__(16) float sm[];
+  const int b = bend - 1 - blockIdx.y, smw = a.wmin << b, ntap = 2 * smw + 1, tid = threadIdx.x;
+  int r;
+  const SmoothBeam &B = row_beam(a, blockIdx.x, &r);
+  if (!*B.active) return;
+  float *const out_s = sm, *const taps = sm + kLC, *const Y = taps + firL_taps(smw);
+  for (int i = tid; i < firL_taps(smw); i += kLT) taps[i] = i < a.tap_n[b] ? a.taps[a.tap_off[b] + i] : 0.f;
+  const YRows rows(B, r, a.ntime_dd);
+  const int H = 2 * smw, org = a.wmax / 2 - (a.anchor ? H : 0), nout = a.ntime_out;
+  const bool vec = rows.vec && (org + H) % 4 == 0 && H % 4 == 0;
+  float *const dst = B.boxes + ((size_t)(b - a.w0) * B.h + r) * nout;
+  float part0 = 0.f, part1 = 0.f, mx = -INFINITY;
+  for (int x = tid; x < H; x += kLT) Y[firL_word(x)] = rows.at(org + x);
+  const float *base = Y + kLPitch * tid;
+  const int nblk = ntap / 16, tail = ntap % 16, key = (tid >> 1) & 3;
+  const float *pcol;  // column 2 tid of the iteration's first 256 in out_s
+  {
+    const int t = tid / 8, q = (tid % 8) / 2;
+    pcol = out_s + 16 * t + 4 * (q ^ ((t >> 1) & 3)) + 2 * (tid & 1);
+  }
+#pragma unroll 1
+  for (int cs = 0; cs < nout; cs += kLC) {
+    const int c0 = cs + org + H;  // columns c0 .. c0 + 2047 enter as y values H .. H + 2047
+    if (vec && c0 >= 0 && c0 + kLC <= rows.n) {
+      float4 x[4], y[4], z[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = c0 + 4 * tid + 4 * kLT * k;
+        x[k] = *reinterpret_cast<const float4 *>(rows.a + c);
+        y[k] = *reinterpret_cast<const float4 *>(rows.b + c);
+        z[k] = *reinterpret_cast<const float4 *>(rows.c + c);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        *reinterpret_cast<float4 *>(Y + firL_word(H + 4 * tid + 4 * kLT * k)) =
+            make_float4(YRows::y(x[k].x, y[k].x, z[k].x), YRows::y(x[k].y, y[k].y, z[k].y),
+                        YRows::y(x[k].z, y[k].z, z[k].z), YRows::y(x[k].w, y[k].w, z[k].w));
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < kLC / kLT; ++k) Y[firL_word(H + tid + kLT * k)] = rows.at(c0 + tid + kLT * k);
+    }
+    __syncthreads();
+    // win[(i + kk) % 16] holds y at window element 16 kq + kk + i of output i; slot kk is refilled
+    // after step kk of block kq
+    float acc[kLO], win[kLO];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 v = *reinterpret_cast<const float4 *>(base + 4 * q);
+      win[4 * q] = v.x, win[4 * q + 1] = v.y, win[4 * q + 2] = v.z, win[4 * q + 3] = v.w;
+    }
+#pragma unroll
+    for (int i = 0; i < kLO; ++i) acc[i] = 0.f;
+    float4 cn = *reinterpret_cast<const float4 *>(taps), yn = *reinterpret_cast<const float4 *>(base + kLPitch);
+    const float *yp = base + kLPitch, *tp = taps;
+#pragma unroll 1
+    for (int kq = 0; kq < nblk; ++kq, yp += kLPitch, tp += 16) {
+#pragma unroll
+      for (int k4 = 0; k4 < 16; k4 += 4) {
+        const float cf[4] = {cn.x, cn.y, cn.z, cn.w}, yv[4] = {yn.x, yn.y, yn.z, yn.w};
+        cn = *reinterpret_cast<const float4 *>(tp + k4 + 4);
+        yn = *reinterpret_cast<const float4 *>(yp + (k4 == 12 ? kLPitch : k4 + 4));
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+#pragma unroll
+          for (int i = 0; i < kLO; ++i) acc[i] = __fmaf_rn(cf[jj], win[(i + k4 + jj) % 16], acc[i]);
+          win[k4 + jj] = yv[jj];
+        }
+      }
+    }
+#pragma unroll
+    for (int k4 = 0; k4 < 16; k4 += 4) {  // the last `tail` taps (no zero taps are issued)
+      if (k4 >= tail) break;
+      const float cf[4] = {cn.x, cn.y, cn.z, cn.w}, yv[4] = {yn.x, yn.y, yn.z, yn.w};
+      if (k4 + 4 < tail) {
+        cn = *reinterpret_cast<const float4 *>(tp + k4 + 4);
+        yn = *reinterpret_cast<const float4 *>(yp + k4 + 4);
+      }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        if (k4 + jj >= tail) break;
+#pragma unroll
+        for (int i = 0; i < kLO; ++i) acc[i] = __fmaf_rn(cf[jj], win[(i + k4 + jj) % 16], acc[i]);
+        win[k4 + jj] = yv[jj];
+      }
+    }
+    if (cs + kLO * tid < nout) {  // nout % 16 == 0
+      store8(dst + cs + kLO * tid, acc);
+      store8(dst + cs + kLO * tid + 8, acc + 8);
+#pragma unroll
+      for (int i = 0; i < kLO; i += 2) mx = max3(mx, acc[i], acc[i + 1]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<float4 *>(out_s + kLO * tid + 4 * (q ^ key)) =
+          make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+    __syncthreads();
+    const int nm = min(kLC / 256, (nout - cs) / 256);  // whole 256s: their columns count for the row mean
+#pragma unroll
+    for (int m = 0; m < kLC / 256; ++m)
+      if (m < nm) {
+        const float2 v = *reinterpret_cast<const float2 *>(pcol + 256 * m);
+        part0 = __fadd_rn(part0, v.x);
+        part1 = __fadd_rn(part1, v.y);
+      }
+    if (cs + kLC < nout) {  // the last H y values move to the front, at most 2048 between barriers
+      for (int x0 = 0; x0 < H; x0 += kLC) {
+        const int n = min(kLC, H - x0);
+        if (H % 4 == 0) {
+          for (int x = x0 + 4 * tid; x < x0 + n; x += 4 * kLT)
+            *reinterpret_cast<float4 *>(Y + firL_word(x)) = *reinterpret_cast<const float4 *>(Y + firL_word(x + kLC));
+        } else {
+          for (int x = x0 + tid; x < x0 + n; x += kLT) Y[firL_word(x)] = Y[firL_word(x + kLC)];
+        }
+        __syncthreads();
+      }
     }
   }
+  __syncthreads();
+  for (int o = 16; o > 0; o /= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  out_s[2 * tid] = part0;
+  out_s[2 * tid + 1] = part1;
+  if ((tid & 31) == 0) out_s[256 + (tid >> 5)] = mx;
+  __syncthreads();
+  if (tid < 32) row_finish(B, b, r, out_s, out_s[256 + (tid & 3)], 256 * (nout / 256));
 }
 
 // Sequential sum of v[0..n) in index order (the reference's host loop),
@@ -762,107 +676,37 @@ __global__ void k_normalise_copy(SmoothArgs a, float *dst) {
 
 }  // namespace
 
-size_t fir_smem_bytes(const SmoothArgs &a) {
-  int ntot = 0;
-  for (int b = a.w0; b < a.w0 + a.nw; ++b) ntot += ((2 * (a.wmin << b) + 1 + kR - 1) / kR) * kR;
-  const int span = 2 * (a.wmin << (a.w0 + a.nw - 1));
-  const int ylen = kCH + span + 2 * kR;
-  const int M = (ylen + kR - 1) / kR;
-  return sizeof(float) * ((size_t)(ntot + 3) / 4 * 4 + (size_t)kR * M + kCH + (size_t)2 * a.nw * kT);
-}
-
-namespace {
-
-// Outputs per thread of k_firR.
-constexpr int kFirR = 16;
-
-// Instantiated phase strides of k_firR (odd, so that staging stores of a
-// warp spread over the banks): spans up to 64, 512 and 2048.
-template <int R>
-struct FirStrides {
-  static constexpr int m0 = (129 + 65 / R) | 1, m1 = (129 + 513 / R) | 1, m2 = (129 + 2049 / R) | 1;
-};
-// Phase stride for the launch's span: the smallest instantiated M >= 129 +
-// (span + 1) / R (the last column the tap loop reads), or 0.
-template <int R>
-int fir_stride(int span) {
-  const int need = 129 + (span + 1) / R;
-  for (int m : {FirStrides<R>::m0, FirStrides<R>::m1, FirStrides<R>::m2})
-    if (need <= m) return m;
-  return 0;
-}
-
-template <int R>
-size_t firR_smem(const SmoothArgs &a, int M) {
-  size_t best = 0;
-  for (int g = 0; g < 2; ++g) {
-    const int wb = g == 0 ? a.w0 : a.split, we = g == 0 ? a.split : a.w0 + a.nw;
-    if (we <= wb) continue;
-    int ntot = 0;
-    for (int b = wb; b < we; ++b) ntot += ((2 * (a.wmin << b) + 1 + 15) / 16) * 16;
-    const size_t f =
-        (size_t)(ntot + 3) / 4 * 4 + (size_t)2 * R * M + (size_t)R * kTF + (size_t)(we - wb) * (256 + kTF);
-    best = std::max(best, f * sizeof(float));
-  }
-  return best;
-}
-
-template <int R, int M>
-cudaError_t launch_firR(const SmoothArgs &a, cudaStream_t s) {
-  const size_t smem = firR_smem<R>(a, M);
-  cudaError_t e = cudaFuncSetAttribute(k_firR<R, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_firR<R, M><<<dim3(a.nrows, a.split < a.w0 + a.nw ? 2 : 1), kTF, smem, s>>>(a);
-  count_launches(1);
-  return cudaGetLastError();
-}
-
-}  // namespace
-
-cudaError_t smooth_planes(const SmoothArgs &a0, cudaStream_t s) {
-  if (a0.nrows <= 0 || a0.nw <= 0) return cudaSuccess;
-  if (a0.wmin == 1 && a0.wmax <= kSSpan && a0.nbox <= kSW && a0.w0 + a0.nw <= kSW && a0.ntime_out % kSO == 0) {
-    const size_t smem = sizeof(float) * ((size_t)kSY + kSW * kSC + kSW * 256 + kSW * kSTap);
-    auto kern = a0.anchor ? k_firS<1> : k_firS<0>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+cudaError_t smooth_planes(const SmoothArgs &a, cudaStream_t s) {
+  if (a.nrows <= 0 || a.nw <= 0) return cudaSuccess;
+  if (a.ntime_out % kLO != 0) return cudaErrorInvalidValue;
+  const int bend = a.w0 + a.nw;
+  // widths 1 .. 32 of a list that starts at 1 go through k_firS, every other width through k_firL
+  // (a width of 32 there: 33 taps for the staging of a chunk of its own)
+  const int bs = a.wmin == 1 ? std::max(a.w0, std::min(bend, kSW)) : a.w0;
+  if (bs < bend) {
+    const int smw = a.wmin << (bend - 1);
+    const size_t smem = sizeof(float) * ((size_t)kLC + firL_taps(smw) + (size_t)firL_rows(smw) * kLPitch);
+    cudaError_t e = cudaFuncSetAttribute(k_firL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<a0.nrows, kST, smem, s>>>(a0);
+    k_firL<<<dim3(a.nrows, bend - bs), kLT, smem, s>>>(a, bend);
+    count_launches(1);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (a.w0 < bs) {
+    SmallTaps t{};
+    for (int b = 0, off = 0; b < std::min(a.nbox, kSW); ++b) {  // padded to multiples of 16 in taps_host
+      const int n = 2 * (1 << b) + 1;
+      std::copy(a.taps_host + off, a.taps_host + off + n, t.t + small_tap(b));
+      off += (n + 15) / 16 * 16;
+    }
+    auto kern = a.anchor ? k_firS<1> : k_firS<0>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSSmem);
+    if (e != cudaSuccess) return e;
+    kern<<<a.nrows, kST, kSSmem, s>>>(a, t, a.w0, bs);
     count_launches(1);
     return cudaGetLastError();
   }
-  SmoothArgs a = a0;
-  a.split = a.w0 + a.nw;
-  const int M = a.ntime_out % kFirR == 0 ? fir_stride<kFirR>(2 * (a.wmin << (a.w0 + a.nw - 1))) : 0;
-  if (M) {
-    // two width groups of about equal taps when the rows alone would leave
-    // the GPU in few waves (fewer than 16 of three blocks per SM)
-    int dev = 0, nsm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      return cudaErrorInvalidDevice;
-    if (a.nw > 1 && a.nrows < 16 * 3 * nsm) {
-      long tot = 0, run = 0, best = -1;
-      for (int b = a.w0; b < a.w0 + a.nw; ++b) tot += 2 * (a.wmin << b) + 1;
-      for (int b = a.w0; b < a.w0 + a.nw - 1; ++b) {
-        run += 2 * (a.wmin << b) + 1;
-        const long worst = std::max(run, tot - run);
-        if (best < 0 || worst < best) {
-          best = worst;
-          a.split = b + 1;
-        }
-      }
-    }
-    using F = FirStrides<kFirR>;
-    if (M == F::m0) return launch_firR<kFirR, F::m0>(a, s);
-    if (M == F::m1) return launch_firR<kFirR, F::m1>(a, s);
-    return launch_firR<kFirR, F::m2>(a, s);
-  }
-  const size_t smem = fir_smem_bytes(a);
-  cudaError_t e = cudaFuncSetAttribute(k_fir, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_fir<<<a.nrows, kT, smem, s>>>(a);
-  count_launches(1);
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 cudaError_t smooth_stats(const SmoothArgs &a, cudaStream_t s, int scale) {
