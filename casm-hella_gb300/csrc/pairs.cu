@@ -7,16 +7,23 @@
 // launches per window:
 //
 // k_pair_build: one block per (group, 4096 window positions for pairs, 2048
-//   for quads).  The group's channels' packed words of the chunk (for
-//   channel i widened by the group's range of relative delays r_i) are read
-//   from the ring once into shared memory as 16-bit lanes (bytes 0 and 2 of
-//   a packed word are the samples p and p + 512), eight loads in flight per
-//   thread, then one warp per row writes every row of the group from them:
-//   row(r)[p] = x[c0][p] + sum_i x[c_i][p + r_i], the next row's metadata
-//   loaded while a row is written.  Reads are the ring once per group;
-//   writes the rows, coalesced, with streaming stores.  A row keeps, tile
-//   by tile, only the words its trials read where those span less than a
-//   1024-sample tile.
+//   for quads).  The group's channels' packed words of the chunk (for channel
+//   i widened by the group's range of relative delays r_i) are bulk-copied
+//   from the ring into shared memory as they are, then one warp per row
+//   writes every row of the group from them: a packed word holds bytes p,
+//   p + 256, p + 512 and p + 768 of a channel, so one read of each channel
+//   gives two words of row(r)[p] = x[c0][p] + sum_i x[c_i][p + r_i], that of
+//   p (bytes 0 and 2) and that of p + 256 (bytes 1 and 3); the next row's
+//   metadata is loaded while a row is written.  Reads are the ring once per
+//   group; writes the rows, coalesced, with streaming stores.  A row keeps,
+//   tile by tile, only the words its trials read where those span less than
+//   a 1024-sample tile.  Bound by the row writes: quads of 2048 channels, DM
+//   0-2000 (14.9 GB) 2.49 ms = 6.0 TB/s, 2.75 ms with the samples split into
+//   16-bit lanes as they were staged (four shared reads a word written, 25
+//   instructions a word against 19); eight beams of 1024 channels 3.28
+//   against 3.91 ms.  Walking positions and keeping the sums over the first
+//   channels from row to row costs more: most blocks of 256 positions are
+//   cut by a row's tile windows (4.88 ms).
 //
 // k_pair_sum: the persistent staging pipeline of k_dedisp (work item =
 //   16-trial tile x 1024 output samples, stages issued warp by warp with
@@ -73,110 +80,141 @@ __device__ __forceinline__ BuildRow build_row(const DedispArgs &a, int r, bool q
   return BuildRow{in.w, in.z, in2.z, in2.w, a.pair_rtile[r], a.pair_rwords[r], a.pair_roff[r]};
 }
 
+// Words of a staged channel window: kBuildCH positions and the channel's range of relative delays,
+// with up to 3 words before (copies start 16-byte aligned) and rounded to whole 16 bytes.
+__host__ __device__ constexpr int build_window(int ch, int span) { return (ch + span + 6) / 4 * 4; }
+
+// One run of up to 256 packed words of a row: output word i takes bytes 0 and 2 of the packed
+// words x[c_i][i], output word i + 256 (i < n2) bytes 1 and 3, for lo <= i < hi.  NC: the group's
+// channels.  With both, the odd bytes are split off and added; the sum of the whole words, in which
+// they sit 8 bits up, less that leaves the even bytes' sums.
+template <int NC, bool BOTH, bool FULL>
+__device__ __forceinline__ void build_run(uint32_t *dst, const uint32_t *sm, const int (&x)[kPairGMax], int lo, int hi,
+                                          int n2) {
+  constexpr int U = 2;  // words of each channel in flight per lane
+#pragma unroll(FULL ? 4 : 1)
+  for (int i0 = (FULL ? 0 : lo) + (threadIdx.x & 31); i0 < (FULL ? 256 : hi); i0 += 32 * U) {
+    uint32_t w[U][NC];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || FULL || i0 + 32 * u < hi)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) w[u][c] = sm[x[c] + i0 + 32 * u];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + 32 * u;
+      const bool in = u == 0 || FULL || i < hi;
+      // rows are read back by other blocks much later: streaming stores
+      if (BOTH) {
+        uint32_t t = w[u][0], o = __byte_perm(w[u][0], 0u, 0x4341);
+#pragma unroll
+        for (int c = 1; c < NC; ++c) t += w[u][c], o += __byte_perm(w[u][c], 0u, 0x4341);
+        if (in) __stcs(dst + i, t - 256u * o);
+        if (FULL || (in && i < n2)) __stcs(dst + 256 + i, o);
+      } else {
+        uint32_t e = w[u][0] & 0x00ff00ffu;
+#pragma unroll
+        for (int c = 1; c < NC; ++c) e += w[u][c] & 0x00ff00ffu;
+        if (in) __stcs(dst + i, e);
+      }
+    }
+  }
+}
+
 template <int G>
-__global__ void __launch_bounds__(256, G == 4 ? 5 : 6) k_pair_build(DedispArgs a) {
-  extern __shared__ uint32_t sm[];
+__global__ void __launch_bounds__(256, G == 4 ? 4 : 5) k_pair_build(DedispArgs a) {
+  extern __shared__ __align__(128) uint32_t sm[];
+  __shared__ __align__(8) unsigned long long bar_s;
+  __shared__ int off_s[kPairGMax];
   constexpr int kBuildCH = build_chunk(G);
   const int k = blockIdx.y, z = blockIdx.z;  // group, beam of the launch
   const long P0 = (long)blockIdx.x * kBuildCH;
   const DedispBeam bm = a.beams ? a.beams[z] : a.one;
   const int r0 = a.pair_prow[k];
   const int r1 = a.pair_rend ? a.pair_rend[(size_t)z * a.pair_npair + k] : a.pair_prow[k + 1];
-  // the group's channels and relative-delay ranges, loaded beside the chunk test's rows
-  const int4 i0 = a.pair_rinfo[r0], j0 = a.pair_rinfo2[r0];
-  int2 rr[kPairGMax];
-  rr[0] = make_int2(0, 0);
-#pragma unroll
-  for (int i = 1; i < kPairGMax; ++i) rr[i] = i < G ? a.pair_prange[k * (kPairGMax - 1) + i - 1] : make_int2(0, 0);
   int any = 0;  // does a row of the group cover a position of this chunk?
   for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     const int w = a.pair_rinfo[r].w;
     any |= P0 < (long)w + row_positions(a, r) && P0 + kBuildCH > (long)w;
   }
   if (!__syncthreads_or(any)) return;
-  const int ch[kPairGMax] = {i0.x, i0.y, G == 4 ? j0.x : -1, G == 4 ? j0.y : -1};  // -1: fewer channels
-  const long R = a.R;
-  // channel i's words for positions [P0 + rmin_i, P0 + kBuildCH + rmax_i) at sm + off[i];
-  // window position p lies at ring word (win0 + p) mod R
-  int off[kPairGMax + 1], rmin[kPairGMax];
-  long base[kPairGMax];
-  int nwin = 0;
-#pragma unroll
-  for (int i = 0; i < kPairGMax; ++i) {
-    off[i] = nwin;
-    rmin[i] = rr[i].x;
-    base[i] = 0;
-    if (i >= G || ch[i] < 0) continue;
-    long b = (bm.win0 + P0 + rr[i].x) % R;
-    base[i] = b < 0 ? b + R : b;
-    nwin += kBuildCH + rr[i].y - rr[i].x;
-  }
-  off[kPairGMax] = nwin;
-  // all the group's windows as one run of words, kLoads ring loads in flight per thread (a
-  // window word's channel: the last i with off[i] <= q; absent channels hold no words)
-  constexpr int kLoads = 8;
-  for (int q0 = threadIdx.x; q0 < nwin; q0 += kLoads * blockDim.x) {
-    uint32_t v[kLoads];
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int q = q0 + u * blockDim.x;
-      if (q < nwin) {
-        int i = 0;
-#pragma unroll
-        for (int j = 1; j < G; ++j) i += q >= off[j] ? 1 : 0;
-        const int c = i == 0 ? ch[0] : i == 1 ? ch[1] : i == 2 ? ch[2] : ch[3];
-        const long b = i == 0 ? base[0] : i == 1 ? base[1] : i == 2 ? base[2] : base[3];
-        const int o = i == 0 ? off[0] : i == 1 ? off[1] : i == 2 ? off[2] : off[3];
-        long pos = b + (q - o);
-        if (pos >= R) pos %= R;
-        v[u] = bm.packed[(size_t)c * R + pos];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int q = q0 + u * blockDim.x;
-      if (q < nwin) sm[q] = __byte_perm(v[u], 0u, 0x4240);
-    }
+  // channel i's packed words for positions [P0 + rmin_i, P0 + kBuildCH + rmax_i), window position p
+  // at ring word (win0 + p) mod R and at sm[off_s[i] + p - P0 + r] for relative delay r: one bulk
+  // copy by lane i, more where the ring wraps
+  const int4 i0 = a.pair_rinfo[r0], j0 = a.pair_rinfo2[r0];
+  const int nc = i0.y < 0 ? 1 : G == 2 || j0.x < 0 ? 2 : j0.y < 0 ? 3 : 4;  // channels of the group
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&bar_s);
+  if (threadIdx.x == 0) {
+    mbar_init(bar, kPairGMax);
+    mbar_fence_init();
   }
   __syncthreads();
-  // one warp per row: the row's metadata is loaded once for 2048-4096 words, the next row's
-  // while this one is written
-  const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  if (threadIdx.x < kPairGMax) {
+    const int i = threadIdx.x;
+    if (i < nc) {
+      const int c = i == 0 ? i0.x : i == 1 ? i0.y : i == 2 ? j0.x : j0.y;
+      const int2 rr = i > 0 ? a.pair_prange[k * (kPairGMax - 1) + i - 1] : make_int2(0, 0);
+      const long R = a.R;  // a multiple of 4, as the copies' ends
+      long pos = (bm.win0 + P0 + rr.x) % R;
+      if (pos < 0) pos += R;
+      const int sh = (int)(pos & 3), len = (sh + kBuildCH + rr.y - rr.x + 3) / 4 * 4;
+      const int at = i * build_window(kBuildCH, a.pair_span);
+      off_s[i] = at + sh - rr.x;
+      pos -= sh;
+      mbar_arrive_tx(bar, 4u * (uint32_t)len);
+      const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(sm);
+      for (int done = 0; done < len;) {
+        const int n = (int)min((long)(len - done), R - pos);
+        bulk_g2s(s0 + 4u * (uint32_t)(at + done), bm.packed + (size_t)c * R + pos, 4u * (uint32_t)n, bar);
+        done += n;
+        pos = 0;
+      }
+    } else {
+      off_s[i] = 0;
+      mbar_arrive(bar);
+    }
+  }
+  __syncthreads();  // off_s
+  if (!mbar_wait(bar, 0)) {
+    if (threadIdx.x == 0 && a.err) atomicOr(a.err, 1);
+    mbar_wait(bar, 0);  // the copies in flight land before the block ends
+    return;
+  }
+  const int of0 = off_s[0], of1 = off_s[1], of2 = off_s[2], of3 = off_s[3];
+  // one warp per row: the row's metadata is loaded once, the next row's while this one is written.
+  // Position first + 512 h + i (i < 256) gives words i and i + 256 of the row's h-th half tile: of
+  // the words of tile h / 2 from 512 (h % 2) on, or of a single run from 512 h on.
+  const int nwarp = blockDim.x >> 5;
   int r = r0 + (threadIdx.x >> 5);
   BuildRow nx{};
   if (r < r1) nx = build_row(a, r, G == 4);
   for (; r < r1; r += nwarp) {
     const BuildRow in = nx;
     if (r + nwarp < r1) nx = build_row(a, r + nwarp, G == 4);
-    const long npos = in.stride == kTileSamples ? (long)in.words : (long)(a.ntt - 1) * kTileSamples + in.stride;
-    if (P0 >= (long)in.w + npos || P0 + kBuildCH <= (long)in.w) continue;
+    const bool run = in.stride == kTileSamples;
+    const int nh = run ? (in.words + 511) / 512 : 2 * a.ntt;
+    const int rel = (int)(P0 - in.w);  // chunk start relative to the row's first position
+    const int h0 = max(0, (rel - 255 + 511) >> 9), h1 = min(nh, (rel + kBuildCH + 511) >> 9);
     uint32_t *dst = a.pair_rows + (size_t)z * a.pair_rows_stride + in.off;
-    // word q of the chunk, q = p - P0, of channel i for this row's r_i
-    const int s1 = off[1] + in.z1 - rmin[1], s2 = off[2] + in.z2 - rmin[2], s3 = off[3] + in.z3 - rmin[3];
-    // the row's tiles: tile tt holds positions [first + 1024 tt, + stride) at words tt * stride on
-    // (one run from word 0 when stride = 1024)
-    const int stride = in.stride;
-    const long rel0 = P0 - in.w;  // chunk start relative to the row's first position
-    const int tt0 = (int)max(0L, rel0 / kTileSamples - 1);
-    const int tt1 = (int)min((long)a.ntt - 1, (rel0 + kBuildCH) / kTileSamples);
-    for (int tt = stride == kTileSamples ? 0 : tt0; tt <= (stride == kTileSamples ? 0 : tt1); ++tt) {
-      // positions of this tile's words (the whole row for stride 1024), clipped to the chunk
-      const long pb = (long)in.w + (long)tt * kTileSamples;
-      const long pe = stride == kTileSamples ? (long)in.w + in.words : pb + stride;
-      const long lo = max(P0, pb), hi = min(P0 + kBuildCH, pe);
-      if (lo >= hi) continue;
-      const int first = (int)(lo - P0), last = (int)(hi - P0);
-      const long d0l = (long)tt * stride + (P0 - pb);  // word of chunk offset q is d0 + q
-      uint32_t *dt = dst + d0l;
-      // rows are read back by other blocks much later: streaming stores
-      if (G == 4 && ch[3] >= 0) {
-        for (int q = first + lane; q < last; q += 32) __stcs(dt + q, sm[q] + sm[s1 + q] + sm[s2 + q] + sm[s3 + q]);
-      } else if (G == 4 && ch[2] >= 0) {
-        for (int q = first + lane; q < last; q += 32) __stcs(dt + q, sm[q] + sm[s1 + q] + sm[s2 + q]);
-      } else if (ch[1] >= 0) {
-        for (int q = first + lane; q < last; q += 32) __stcs(dt + q, sm[q] + sm[s1 + q]);
+    const int s0 = of0, s1 = of1 + in.z1, s2 = of2 + in.z2, s3 = of3 + in.z3;
+    for (int h = h0; h < h1; ++h) {
+      const int q = 512 * h - rel;  // chunk offset of the half tile's first position
+      const int left = run ? in.words - 512 * h : in.stride - 512 * (h & 1);
+      if (left <= 0) continue;
+      uint32_t *d = dst + (run ? 512 * h : (h >> 1) * in.stride + 512 * (h & 1));
+      const int lo = max(0, -q), n2 = min(256, left - 256), hi = min(min(256, left), kBuildCH - q);
+      const int x[kPairGMax] = {s0 + q, s1 + q, s2 + q, s3 + q};
+      const bool full = lo == 0 && hi == 256 && n2 == 256;
+      if (nc == G) {
+        if (full) build_run<G, true, true>(d, sm, x, lo, hi, n2);
+        else if (n2 > lo) build_run<G, true, false>(d, sm, x, lo, hi, n2);
+        else build_run<G, false, false>(d, sm, x, lo, hi, n2);
+      } else if (G == 4 && nc == 3) {  // the last group
+        build_run<3, true, false>(d, sm, x, lo, hi, n2);
+      } else if (G == 4 && nc == 2) {
+        build_run<2, true, false>(d, sm, x, lo, hi, n2);
       } else {
-        for (int q = first + lane; q < last; q += 32) __stcs(dt + q, sm[q]);
+        build_run<1, true, false>(d, sm, x, lo, hi, n2);
       }
     }
   }
@@ -616,7 +654,7 @@ cudaError_t dedisperse_pairs(const DedispArgs &a, cudaStream_t s) {
   if (a.R <= 0 || (!a.beams && a.one.win0 < 0)) return cudaErrorInvalidValue;
   // the group's channel windows: ch words for c0, ch + its r range for the others
   const int ch = build_chunk(g);
-  const size_t bsmem = ((size_t)g * ch + (size_t)(g - 1) * a.pair_span) * 4;
+  const size_t bsmem = (size_t)g * build_window(ch, a.pair_span) * 4;
   if (bsmem > 200 * 1024) return cudaErrorInvalidValue;
   auto kern = g == 4 ? k_pair_build<4> : k_pair_build<2>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem);
