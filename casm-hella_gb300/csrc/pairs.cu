@@ -33,13 +33,16 @@
 //   thread j then reads, per group and trial, the words j and j + 256 of
 //   the trial's window: four output samples (j, j+256, j+512, j+768) in two
 //   SWAR registers of 16-bit lanes, two groups per three-input add.  The
-//   lanes are widened into 32-bit totals every pair_lanecap(g) groups.
+//   lanes are widened into 32-bit totals, held in tensor memory, every
+//   pair_lanecap(g) groups.
 //
 // Per group and trial the inner loop is two shared loads and one add for
 // 4g channel-samples, against two loads, four byte permutes and two adds
 // per eight in k_dedisp; shared-memory traffic is 2/g bytes per
-// channel-sample, so the sums are bound by shared-memory bandwidth, and
-// the build by its row writes (g = 4: about three times the rows of g = 2).
+// channel-sample, so the sums are bound by shared-memory bandwidth (reads
+// and staged rows at 80 to 93 % of its cycles), quads by the rows' latency as
+// well (with nothing staged 5.8 of 7.4 ms), and the build by its row writes
+// (g = 4: about three times the rows of g = 2).
 #include "hg_internal.h"
 #include "hg_ptx.h"
 
@@ -55,9 +58,18 @@ constexpr int kTileSamples = 4 * S;
 // window positions per build block: 4096 for pairs, 2048 for quads (whose
 // four channel windows would otherwise leave three blocks per SM)
 __host__ __device__ constexpr int build_chunk(int g) { return g <= 2 ? 4096 : 2048; }
+constexpr int kTmemAt = 440;              // the block's tensor memory address, in the first unit's header
 constexpr int kBarHdr = 448;              // full[4] | empty[4] | per-warp staging cursors
-constexpr size_t kSmemBudget = 113 * 1024;  // two resident blocks per SM (228 KB less 1 KB a block)
+constexpr size_t kSmemMost = 227 * 1024;  // of a block, one to an SM
 constexpr int kMaxBuf = 4;
+
+// Shared memory of one unit of the sum (half a block): barriers and cursors, staging buffers.
+__host__ __device__ constexpr size_t unit_smem(int bufbytes, int nbuf) { return kBarHdr + (size_t)nbuf * bufbytes; }
+
+// Words of a copy that only outputs past the last one would read: the last time tile's `rem`
+// outputs need the words j < rem alone when they are at most 512 (word j + 256 holds outputs
+// j + 256 and j + 768).
+__host__ __device__ constexpr int words_cut(int rem) { return rem < 2 * S ? 2 * S - (rem + 3) / 4 * 4 : 0; }
 
 __host__ __device__ constexpr int stage_hdr_bytes(int cc) { return 16 + cc * kPairDPT * 4; }
 
@@ -181,6 +193,7 @@ __global__ void __launch_bounds__(256, G == 4 ? 4 : 5) k_pair_build(DedispArgs a
     return;
   }
   const int of0 = off_s[0], of1 = off_s[1], of2 = off_s[2], of3 = off_s[3];
+  const int cut = words_cut(a.nout - (a.ntt - 1) * kTileSamples);  // words of the last tile nobody reads
   // one warp per row: the row's metadata is loaded once, the next row's while this one is written.
   // Position first + 512 h + i (i < 256) gives words i and i + 256 of the row's h-th half tile: of
   // the words of tile h / 2 from 512 (h % 2) on, or of a single run from 512 h on.
@@ -192,14 +205,14 @@ __global__ void __launch_bounds__(256, G == 4 ? 4 : 5) k_pair_build(DedispArgs a
     const BuildRow in = nx;
     if (r + nwarp < r1) nx = build_row(a, r + nwarp, G == 4);
     const bool run = in.stride == kTileSamples;
-    const int nh = run ? (in.words + 511) / 512 : 2 * a.ntt;
+    const int total = in.words - cut, nh = run ? (total + 511) / 512 : 2 * a.ntt;
     const int rel = (int)(P0 - in.w);  // chunk start relative to the row's first position
     const int h0 = max(0, (rel - 255 + 511) >> 9), h1 = min(nh, (rel + kBuildCH + 511) >> 9);
     uint32_t *dst = a.pair_rows + (size_t)z * a.pair_rows_stride + in.off;
     const int s0 = of0, s1 = of1 + in.z1, s2 = of2 + in.z2, s3 = of3 + in.z3;
     for (int h = h0; h < h1; ++h) {
       const int q = 512 * h - rel;  // chunk offset of the half tile's first position
-      const int left = run ? in.words - 512 * h : in.stride - 512 * (h & 1);
+      const int left = run ? total - 512 * h : in.stride - 512 * (h & 1) - (h >> 1 == a.ntt - 1 ? cut : 0);
       if (left <= 0) continue;
       uint32_t *d = dst + (run ? 512 * h : (h >> 1) * in.stride + 512 * (h & 1));
       const int lo = max(0, -q), n2 = min(256, left - 256), hi = min(min(256, left), kBuildCH - q);
@@ -220,34 +233,52 @@ __global__ void __launch_bounds__(256, G == 4 ? 4 : 5) k_pair_build(DedispArgs a
   }
 }
 
-__device__ __forceinline__ void pair_item(const DedispArgs &a, int ntiles, int l, int *tile, int *tt) {
-  const int per_group = a.group * a.ntt;
+// Tile and time tile of item l of a beam's, over its first `ntt` time tiles: `group` DM tiles a time
+// tile together.
+__device__ __forceinline__ void pair_item(const DedispArgs &a, int ntiles, int ntt, int l, int *tile, int *tt) {
+  const int per_group = a.group * ntt;
   const int g = l / per_group, r = l - g * per_group;
   const int gsz = min(a.group, ntiles - g * a.group);
   *tt = r / gsz;
   *tile = g * a.group + (r - *tt * gsz);
 }
 
+// A block is two units of 256 threads (one where work or shared memory is for
+// one), each with staging buffers, barriers and work items of its own: one
+// block an SM, because the totals live in tensor memory and blocks that hold
+// some do not share an SM (two 256-thread blocks ran one after the other).
+// The 64 totals a thread would otherwise keep in registers are touched once
+// in 64 quads; without them the shared reads of several trials are in flight
+// at once.  Eight beams of 1024 channels (quads): 7.45 ms against 7.89 with
+// the totals in registers (7.75 once a stage's record is prefetched), 16
+// beams' short gulps (pairs) 6.18 against 6.30, 2048 channels to DM 2000 the
+// same 6.9 ms; lanes added into the output plane instead (red.add every 57
+// quads) 9.5 ms there.  Tiles of 32 trials, two units summing 16 each from the
+// same staged rows, stage 30 % less and are slower (7.74, 6.37, 7.08 ms).
 // MULTI: the launch serves several beams (a.beams, batched context): each
 // item looks up its beam; else the one beam's record stays in registers.
 template <int CC, bool MULTI>
-__global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, int bufbytes, int nbuf) {
+__global__ void __launch_bounds__(2 * kDedispThreads, 1) k_pair_sum(DedispArgs a, int bufbytes, int nbuf) {
   extern __shared__ __align__(128) uint32_t smem[];
   constexpr int DPT = kPairDPT;
   constexpr int NWARP = kDedispThreads / 32;
   constexpr int HB = stage_hdr_bytes(CC);
+  constexpr uint32_t kTotCols = 256;  // four warps' 64 totals a lane
   const int REC = pair_rec_int4(CC);
-  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+  const int half = threadIdx.x / kDedispThreads, unit = blockIdx.x * (blockDim.x / kDedispThreads) + half;
+  const int units = gridDim.x * (blockDim.x / kDedispThreads);
+  char *const mine = reinterpret_cast<char *>(smem) + (size_t)half * unit_smem(bufbytes, nbuf);
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(mine);
   auto full_of = [&](int b) { return sbase + 8u * b; };
   auto empty_of = [&](int b) { return sbase + 32u + 8u * b; };
   auto buf_of = [&](int b) { return sbase + kBarHdr + (uint32_t)b * (uint32_t)bufbytes; };
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x % kDedispThreads, lane = tid & 31, warp = tid >> 5;
   // the stage a warp stages next: stage st of the nst stages of block-local item k
   struct Cursor {
     int k, st, s0, nst, t0, z;  // z: beam of the item in the launch
   };
-  static_assert(64 + NWARP * sizeof(Cursor) <= kBarHdr, "staging cursors");
-  Cursor *cur = reinterpret_cast<Cursor *>(reinterpret_cast<char *>(smem) + 64) + warp;
+  static_assert(64 + NWARP * sizeof(Cursor) <= kTmemAt, "staging cursors");
+  Cursor *cur = reinterpret_cast<Cursor *>(mine + 64) + warp;
   if (tid == 0) {
     for (int b = 0; b < nbuf; ++b) {
       mbar_init(full_of(b), 32);      // every lane of the staging warp arrives once per fill
@@ -255,28 +286,40 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, in
     }
     mbar_fence_init();
   }
+  if (threadIdx.x < 32) tmem_alloc((uint32_t)__cvta_generic_to_shared(smem) + kTmemAt, kTotCols);
   __syncthreads();
-  if (blockIdx.x >= a.nitems) return;
+  // this thread's 64 totals: columns 4 m + k (trial m, sample j + 256 k)
+  const uint32_t tmem = smem[kTmemAt / 4];
+  const uint32_t totals = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(threadIdx.x >> 7) * 64u;
 
-  // Beam z of launch item `item` and the item's tile and time tile: the
-  // items of the launch's beams follow one another (beam z's from
-  // beams[z].item0 - beams[0].item0 on; a beam without trials has none).
+  // Beam z of launch item `item` and the item's tile and time tile.  A last
+  // time tile that only needs part of its words (words_cut; outputs past a
+  // gulp of whole tiles are the smoothing's few) makes a short item: those of
+  // all tiles and beams come last and fill the last round, which whole items
+  // would mostly leave empty (16 beams x 8256 outputs 6.23 -> 5.95 ms).  Beam z's tiles are the launch's from (beams[z].
+  // item0 - beams[0].item0) / ntt on; a beam without trials has none.
   const DedispBeam b0 = MULTI ? a.one : (a.beams ? a.beams[0] : a.one);
+  const int nlong = words_cut(a.nout - (a.ntt - 1) * kTileSamples) > 0 && a.ntt > 1 ? a.ntt - 1 : a.ntt;
+  const int shorts = a.nitems / a.ntt * nlong;  // first short item
   auto locate = [&](int item, int *z, int *tile, int *tt) -> DedispBeam {
+    const bool tail = item >= shorts;
+    const int per = tail ? 1 : nlong;  // items of a tile
+    if (tail) item -= shorts;
     int zz = 0;
     DedispBeam bz = b0;
     if (MULTI) {
-      const int g = a.beams[0].item0 + item;
-      while (zz + 1 < a.nbeam && a.beams[zz + 1].item0 <= g) ++zz;
+      const int i0 = a.beams[0].item0;
+      while (zz + 1 < a.nbeam && (a.beams[zz + 1].item0 - i0) / a.ntt * per <= item) ++zz;
       bz = a.beams[zz];
-      item = g - bz.item0;
+      item -= (bz.item0 - i0) / a.ntt * per;
     }
     *z = zz;
-    pair_item(a, (bz.dm_count + DPT - 1) / DPT, item, tile, tt);
+    pair_item(a, (bz.dm_count + DPT - 1) / DPT, per, item, tile, tt);
+    if (tail) *tt = a.ntt - 1;
     return bz;
   };
   auto load_item = [&](int k) -> bool {  // lane 0
-    const int item = blockIdx.x + k * gridDim.x;
+    const int item = unit + k * units;
     if (item >= a.nitems) return false;
     int z, tile, tt;
     locate(item, &z, &tile, &tt);
@@ -301,6 +344,13 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, in
     p_done = !__shfl_sync(0xffffffffu, more, 0);
     __syncwarp();
   }
+  // the record of the warp's next stage on its way to L1: the staging warp would otherwise sit out
+  // two loads from L2 or DRAM, and the unit with it
+  auto prefetch = [&]() {
+    const int4 *r = a.pair_rec + (size_t)(cur->s0 + cur->st) * REC;
+    prefetch_l1(lane == 31 ? r : r + 1 + CC * DPT / 4 + lane);
+  };
+  if (!p_done) prefetch();
   auto issue = [&](bool block, bool *timed_out) -> bool {
     const unsigned g = g_next;
     const int b = (int)(g % (unsigned)nbuf);
@@ -324,7 +374,8 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, in
       // {first word (low, high), words | byte slot / 16 << 16, the row's words per time tile}
       const int4 rw = __ldg(r + 1 + CC * DPT / 4 + lane);
       const long start = (long)(((unsigned long long)(unsigned)rw.y << 32) | (unsigned)rw.x);
-      const uint32_t nb = ((uint32_t)rw.z & 0xffffu) * 4u, slot = ((uint32_t)rw.z >> 16) * 16u;
+      const uint32_t nb = (((uint32_t)rw.z & 0xffffu) - (uint32_t)words_cut(a.nout - cur->t0)) * 4u,
+                     slot = ((uint32_t)rw.z >> 16) * 16u;
       mbar_arrive_tx(bar, nb + (lane == 0 ? (uint32_t)HB : 0u));
       const uint32_t *rows = MULTI ? a.pair_rows + (size_t)cur->z * a.pair_rows_stride : a.pair_rows;
       bulk_g2s(buf_of(b) + HB + slot, rows + start + (long)tt * rw.w, nb, bar);
@@ -338,6 +389,7 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, in
     if (lane == 0) more = advance(NWARP);
     p_done = !__shfl_sync(0xffffffffu, more, 0);
     __syncwarp();
+    if (!p_done) prefetch();
     return true;
   };
   // After a wait ran out: record it, let this warp's copies land, end.
@@ -348,27 +400,47 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, in
   };
 
   unsigned gs_c = 0;  // stages consumed
-  for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
+  bool ok = true;     // no wait of this warp ran out
+  for (int item = unit; ok && item < a.nitems; item += units) {
     int z, tile, tt;
     const DedispBeam bm = locate(item, &z, &tile, &tt);
+    // what of the warp's outputs there is in the last time tile: words j (any), words j + 256
+    const int rem = a.nout - tt * kTileSamples - 32 * warp;
+    const bool any = rem > 0, both = rem > S;
     const int nstage = a.pair_tile_st[tile + 1] - a.pair_tile_st[tile];
-    uint32_t acc_a[DPT], acc_b[DPT], tot[DPT][4];  // acc_a: samples j, j+512; acc_b: j+256, j+768
+    uint32_t acc_a[DPT], acc_b[DPT];  // acc_a: samples j, j+512; acc_b: j+256, j+768
 #pragma unroll
-    for (int m = 0; m < DPT; ++m) {
-      acc_a[m] = acc_b[m] = 0u;
+    for (int m = 0; m < DPT; ++m) acc_a[m] = acc_b[m] = 0u;
+    bool stored = false;  // the totals hold the lanes of earlier stages
+    auto widen = [&](uint32_t (&v)[4 * DPT]) {
+      if (stored) {
+        tmem_ld64(totals, v);
+      } else {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) tot[m][k] = 0u;
-    }
+        for (int i = 0; i < 4 * DPT; ++i) v[i] = 0u;
+      }
+#pragma unroll
+      for (int m = 0; m < DPT; ++m) {
+        v[4 * m] += acc_a[m] & 0xffffu;
+        v[4 * m + 1] += acc_b[m] & 0xffffu;
+        v[4 * m + 2] += acc_a[m] >> 16;
+        v[4 * m + 3] += acc_b[m] >> 16;
+      }
+    };
     int npairs = 0;  // groups in the 16-bit lanes
     for (int st = 0; st < nstage; ++st) {
       {
         bool to = false;
         while (!p_done && g_next < gs_c + nbuf)
           if (!issue(g_next <= gs_c, &to)) break;
-        if (to) return fail(gs_c);
+        const int b = (int)(gs_c % (unsigned)nbuf);
+        if (to || !mbar_wait(full_of(b), (gs_c / nbuf) & 1u)) {
+          fail(gs_c);
+          ok = false;
+          break;
+        }
       }
       const int b = (int)(gs_c % (unsigned)nbuf);
-      if (!mbar_wait(full_of(b), (gs_c / nbuf) & 1u)) return fail(gs_c);
       const uint32_t hb = buf_of(b), ob = hb + 16u, rb = hb + (uint32_t)HB + (uint32_t)tid * 4u;
       const int ng = (int)lds32(hb);
       auto add2 = [&](int i) {  // pairs i and i + 1
@@ -400,37 +472,38 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, in
           }
         }
       };
-      if (ng == CC) {
-#pragma unroll
-        for (int i = 0; i < CC; i += 2) add2(i);
-      } else {
+      if (both) {
         int i = 0;
         for (; i + 1 < ng; i += 2) add2(i);
         if (i < ng) add1(i);
+      } else if (any) {
+        for (int i = 0; i < ng; ++i)
+#pragma unroll
+          for (int q = 0; q < DPT / 4; ++q) {
+            const int4 x1 = lds128(ob + (uint32_t)(i * DPT + 4 * q) * 4u);
+            acc_a[4 * q] += lds32(rb + (uint32_t)x1.x);
+            acc_a[4 * q + 1] += lds32(rb + (uint32_t)x1.y);
+            acc_a[4 * q + 2] += lds32(rb + (uint32_t)x1.z);
+            acc_a[4 * q + 3] += lds32(rb + (uint32_t)x1.w);
+          }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty_of(b));  // this warp is done with buffer b
       ++gs_c;
       npairs += ng;
       if (npairs + CC > a.pair_lanecap) {
+        uint32_t v[4 * DPT];
+        widen(v);
+        tmem_st64(totals, v);
+        stored = true;
 #pragma unroll
-        for (int m = 0; m < DPT; ++m) {
-          tot[m][0] += acc_a[m] & 0xffffu;
-          tot[m][2] += acc_a[m] >> 16;
-          tot[m][1] += acc_b[m] & 0xffffu;
-          tot[m][3] += acc_b[m] >> 16;
-          acc_a[m] = acc_b[m] = 0u;
-        }
+        for (int m = 0; m < DPT; ++m) acc_a[m] = acc_b[m] = 0u;
         npairs = 0;
       }
     }
-#pragma unroll
-    for (int m = 0; m < DPT; ++m) {
-      tot[m][0] += acc_a[m] & 0xffffu;
-      tot[m][2] += acc_a[m] >> 16;
-      tot[m][1] += acc_b[m] & 0xffffu;
-      tot[m][3] += acc_b[m] >> 16;
-    }
+    if (!ok) break;
+    uint32_t v[4 * DPT];
+    widen(v);
     const int t0 = tt * kTileSamples;
 #pragma unroll
     for (int m = 0; m < DPT; ++m) {
@@ -440,37 +513,39 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_pair_sum(DedispArgs a, in
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int t = t0 + tid + k * S;
-        if (t < a.nout) o[t] = (float)tot[m][k];
+        if (t < a.nout) o[t] = (float)v[4 * m + k];
       }
     }
   }
+  tmem_wait_st();
+  __syncthreads();
+  if (threadIdx.x < 32) tmem_free(tmem, kTotCols);
 }
 
 template <int CC, bool MULTI>
 cudaError_t launch_sum(const DedispArgs &a, cudaStream_t s) {
   const int bufbytes = stage_hdr_bytes(CC) + a.pair_stage;
+  // the pipeline asked for, else the deepest that leaves room for two units; two buffers at least
+  const size_t share = kSmemMost / 2 / 16 * 16;
   int nbuf = a.nbuf;
-  if (!nbuf) {  // deepest pipeline within the two-blocks budget, else two buffers
-    nbuf = 2;
-    for (int nb = kMaxBuf; nb >= 2; --nb)
-      if (kBarHdr + (size_t)nb * bufbytes <= kSmemBudget) {
-        nbuf = nb;
-        break;
-      }
+  if (!nbuf) {
+    nbuf = kMaxBuf;
+    while (nbuf > 2 && unit_smem(bufbytes, nbuf) > share) --nbuf;
   }
   if (nbuf < 2 || nbuf > kMaxBuf) return cudaErrorInvalidValue;
-  const size_t smem = kBarHdr + (size_t)nbuf * bufbytes;
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;
-  auto kern = k_pair_sum<CC, MULTI>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t one = unit_smem(bufbytes, nbuf);
+  if (one > kSmemMost) return cudaErrorInvalidValue;
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 0, per_sm = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kDedispThreads, smem)) != cudaSuccess)
+  // units per block: two where they fit, unless each item can have an SM of its own
+  const int halves = one <= share && a.nitems > sms ? 2 : 1;
+  auto kern = k_pair_sum<CC, MULTI>;
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(halves * one))) != cudaSuccess)
     return e;
-  const int grid = std::max(1, std::min(a.nitems, std::max(1, per_sm) * sms));
-  kern<<<grid, kDedispThreads, smem, s>>>(a, bufbytes, nbuf);
+  const int grid = std::max(1, std::min((a.nitems + halves - 1) / halves, sms));
+  kern<<<grid, halves * kDedispThreads, halves * one, s>>>(a, bufbytes, nbuf);
   count_launches(1);
   return cudaGetLastError();
 }
