@@ -10,10 +10,13 @@
 // of every DM trial in the block's tile, so for channel c and trial d it
 // reads the single word at t0 + j + delay(c,d): 32 lanes read 32
 // consecutive words (no bank conflicts) whatever the delay, and each 4-byte
-// read feeds four sums.  The bytes are split into two SWAR registers of
-// 16-bit lanes with byte_perm (samples k=0,2 and k=1,3); two channels are
-// added per three-input add.  256 channels of u8 fit a 16-bit lane
-// (255*256 < 2^16), after which the lanes are widened into 32-bit totals.
+// read feeds four sums: the words are added as they are (mod 2^32), and
+// their odd bytes (samples k=1,3), split off with byte_perm, as 16-bit lanes;
+// two channels are added per three-input add.  The odd sums 8 bits up taken
+// from the words' sum leave the even bytes' (k=0,2), so a word costs one byte
+// permute, not two: 512 channels x 495 trials x 16448 samples 245 us against
+// 295.  256 channels of u8 fit a 16-bit lane (255*256 < 2^16), after which
+// the lanes are widened into 32-bit totals.
 //
 // Staging.  A work item is (beam, tile of DPT trials, 4S samples); the
 // block walks the tables' channels CC at a time.  Host-built tile tables
@@ -121,14 +124,25 @@ __device__ __forceinline__ Item item_at(const DedispArgs &a, int item) {
   return it;
 }
 
+// Totals of samples k = 0..3 from the sums of whole words (mod 2^32) and of
+// their odd bytes (16-bit lanes): the odd bytes sit 8 bits up in the words,
+// and what is left without them are the even bytes' sums, as long as each
+// stays below 2^16.
+__device__ __forceinline__ void widen(uint32_t (&tot)[4], uint32_t w, uint32_t o) {
+  const uint32_t e = w - (o << 8);
+  tot[0] += e & 0xffffu;
+  tot[2] += e >> 16;
+  tot[1] += o & 0xffffu;
+  tot[3] += o >> 16;
+}
+
 // MODE picks how the integer adds are spread over the SM's pipes (the
 // sums are identical): 0 = three-input adds throughout; 1 = load addresses
 // as multiply-adds by a runtime 1 (FMA pipe); 2 = as 1, and the odd-sample
 // lanes accumulated by multiply-adds as well; 3 = two-input address adds
 // (which issue on the full-rate FMA pipes), odd lanes by multiply-adds.
 // Byte permutes and three-input adds share the half-rate ALU pipe, and
-// multiply-adds the half-rate heavy FMA pipe, so MODE 3 leaves 2.5 ALU
-// and 2 multiply-add instructions per word.
+// multiply-adds the half-rate heavy FMA pipe.
 //
 // VAR: the launch's items differ in their number of stages (beams with
 // tables of their own), so each warp walks a cursor over the items; else
@@ -301,10 +315,10 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_dedisp(DedispArgs a, int 
   for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
     const int nact = VAR ? item_nact(a, item) : a.nact;
     const int nstage = VAR ? (nact + CC - 1) / CC : nstage_u;
-    uint32_t acc_e[DPT], acc_o[DPT], tot[DPT][4];
+    uint32_t acc_w[DPT], acc_o[DPT], tot[DPT][4];  // whole words; odd bytes as 16-bit lanes
 #pragma unroll
     for (int m = 0; m < DPT; ++m) {
-      acc_e[m] = acc_o[m] = 0u;
+      acc_w[m] = acc_o[m] = 0u;
 #pragma unroll
       for (int k = 0; k < 4; ++k) tot[m][k] = 0u;
     }
@@ -336,7 +350,7 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_dedisp(DedispArgs a, int 
               constexpr bool kMadAddr = MODE == 1 || MODE == 2;
               const uint32_t w1 = lds32(kMadAddr ? (uint32_t)o1[j] * unit + r1 : r1 + (uint32_t)o1[j]);
               const uint32_t w2 = lds32(kMadAddr ? (uint32_t)o2[j] * unit + r2 : r2 + (uint32_t)o2[j]);
-              acc_e[m] += __byte_perm(w1, 0u, 0x4240) + __byte_perm(w2, 0u, 0x4240);
+              acc_w[m] += w1 + w2;
               if (MODE >= 2) {
                 acc_o[m] = __byte_perm(w1, 0u, 0x4341) * unit + acc_o[m];
                 acc_o[m] = __byte_perm(w2, 0u, 0x4341) * unit + acc_o[m];
@@ -358,7 +372,7 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_dedisp(DedispArgs a, int 
             const int m = 4 * q + j;
             if (m < DPT) {
               const uint32_t w1 = lds32(r1 + (uint32_t)o1[j]);
-              acc_e[m] += __byte_perm(w1, 0u, 0x4240);
+              acc_w[m] += w1;
               acc_o[m] += __byte_perm(w1, 0u, 0x4341);
             }
           }
@@ -378,21 +392,13 @@ __global__ void __launch_bounds__(kDedispThreads, 2) k_dedisp(DedispArgs a, int 
       if ((st + 1) % (256 / CC) == 0) {  // 256 channels per 16-bit lane, then widen
 #pragma unroll
         for (int m = 0; m < DPT; ++m) {
-          tot[m][0] += acc_e[m] & 0xffffu;
-          tot[m][2] += acc_e[m] >> 16;
-          tot[m][1] += acc_o[m] & 0xffffu;
-          tot[m][3] += acc_o[m] >> 16;
-          acc_e[m] = acc_o[m] = 0u;
+          widen(tot[m], acc_w[m], acc_o[m]);
+          acc_w[m] = acc_o[m] = 0u;
         }
       }
     }
 #pragma unroll
-    for (int m = 0; m < DPT; ++m) {
-      tot[m][0] += acc_e[m] & 0xffffu;
-      tot[m][2] += acc_e[m] >> 16;
-      tot[m][1] += acc_o[m] & 0xffffu;
-      tot[m][3] += acc_o[m] >> 16;
-    }
+    for (int m = 0; m < DPT; ++m) widen(tot[m], acc_w[m], acc_o[m]);
     const Item it = item_at<DPT>(a, item);
 #pragma unroll
     for (int m = 0; m < DPT; ++m) {
@@ -825,7 +831,7 @@ size_t dedisp_smem_bytes(int dpt, int cc, int max_spread) {
 }
 
 DedispTables dedisp_tables(const int *delays, int nchan, const int *chans, int nact, int dm_first,
-                           int dm_count, int dpt, int cc) {
+                           int dm_count, int dpt, int cc, int dpt_max) {
   DedispTables t;
   const int dlast = dm_first + dm_count - 1;
   if (dpt > 0) {
@@ -833,6 +839,7 @@ DedispTables dedisp_tables(const int *delays, int nchan, const int *chans, int n
     t.max_spread = dedisp_spread(delays, nchan, chans, nact, dm_first, dm_count, dpt);
   } else {
     for (int d : {16, 8, 4, 2, 1}) {
+      if (d > dpt_max) continue;
       const int spread = dedisp_spread(delays, nchan, chans, nact, dm_first, dm_count, d);
       if (dedisp_smem_bytes(d, cc, spread) || d == 1) {
         t.dpt = d;

@@ -166,6 +166,16 @@ cudaError_t gather_tables(const int4 *meta, const int *off, int nch, int dpt, co
                           int max_tiles, const int *chans, int4 *bmeta, int *boff, cudaStream_t s);
 // Work items of one beam for a tile shape.
 inline int dedisp_items(int dm_count, int dpt, int ntt) { return (dm_count + dpt - 1) / dpt * ntt; }
+// Largest tile worth taking for a launch of `count` trials over ntt time
+// tiles, not below `least`: halved while its items would leave SMs without
+// one, where a stage's time is the latency of its few adds (143 trials x 1501
+// samples x 128 channels: 27.2 us with 18 items of 16 trials, 19.6 with 72 of 4, 18.9 with
+// 144 of 2).
+inline int dedisp_tile_cap(int count, int ntt, int least) {
+  int d = 16;
+  while (d > least && dedisp_items(count, d, ntt) < 152) d /= 2;
+  return d;
+}
 inline int dedisp_time_tiles(int nout) { return (nout + 4 * kPackS - 1) / (4 * kPackS); }
 // Launches the persistent kernel over all items of `a`.
 cudaError_t dedisperse(const DedispArgs &a, cudaStream_t s);
@@ -176,15 +186,16 @@ size_t dedisp_smem_bytes(int dpt, int cc, int max_spread);
 int dedisp_nbuf(int dpt, int cc, int max_spread);
 
 // Host-side tile tables for trials [dm_first, dm_first + dm_count) over the
-// active channels, for `dpt` trials per tile (dpt = 0: the largest tile
-// whose double-buffered staging of cc channels fits in shared memory).
+// active channels, for `dpt` trials per tile (dpt = 0: the largest tile of
+// at most dpt_max trials whose double-buffered staging of cc channels fits in
+// shared memory).
 struct DedispTables {
   int dpt = 0, max_spread = 0, ntiles = 0, offw = 0;
   std::vector<int4> meta;
   std::vector<int> off;
 };
 DedispTables dedisp_tables(const int *delays_host, int nchan, const int *chans_host, int nact,
-                           int dm_first, int dm_count, int dpt = 0, int cc = 8);
+                           int dm_first, int dm_count, int dpt = 0, int cc = 8, int dpt_max = 16);
 // Tables of add mode 4 (sub-band sums shared by a 16-trial tile's trials,
 // groups of four consecutive active channels); meta as DedispTables.meta
 // for 16-trial tiles.

@@ -14,16 +14,16 @@ std::vector<float> delay_table(int nchan, double dt_s, double f0, double df);
 std::vector<int> dm_delays(const std::vector<float> &dms, const std::vector<float> &table);
 
 // Dedispersion tile tables for trials [first, first + count) with dpt
-// trials per tile (0: the largest that fits cc-channel stages): host copy
+// trials per tile (0: the largest up to dpt_max that fits cc-channel stages): host copy
 // (cached per range and shape) and device copy (uploaded on first use).
-const DedispTables &plan_host_tables(hdd_plan p, int first, int count, int dpt = 0, int cc = 8);
+const DedispTables &plan_host_tables(hdd_plan p, int first, int count, int dpt = 0, int cc = 8, int dpt_max = 16);
 struct DeviceTables {
   const int4 *meta;
   const int *off;
   int dpt, max_spread, nact, cc;
 };
 hdd_error plan_device_tables(hdd_plan p, int first, int count, DeviceTables *out, int dpt = 0,
-                             int cc = 8);
+                             int cc = 8, int dpt_max = 16);
 // Add-mode-4 tables for trials [first, first + count) over the plan's
 // active channels: host copy cached per range, device copy uploaded on first use.
 struct SubDeviceTables {

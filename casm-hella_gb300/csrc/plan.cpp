@@ -84,7 +84,7 @@ struct hdd_plan_struct {
   int max_delay = 0;
   // dedispersion tile tables of the last DM range used, host and device
   hg::DedispTables tab;
-  int tab_first = -1, tab_count = -1, tab_dpt = -1, tab_cc = -1;
+  int tab_first = -1, tab_count = -1, tab_dpt = -1, tab_cc = -1, tab_max = -1;
   bool tab_on_device = false;
   int *d_err = nullptr;  // dedispersion status word
   int4 *d_meta = nullptr;
@@ -175,10 +175,13 @@ hdd_error grow(void **ptr, size_t *cap, size_t need) {
 
 namespace hg {
 
-const DedispTables &plan_host_tables(hdd_plan p, int first, int count, int dpt, int cc) {
-  if (p->tab_first != first || p->tab_count != count || p->tab_dpt != dpt || p->tab_cc != cc) {
+const DedispTables &plan_host_tables(hdd_plan p, int first, int count, int dpt, int cc, int dpt_max) {
+  if (dpt > 0) dpt_max = 16;
+  if (p->tab_first != first || p->tab_count != count || p->tab_dpt != dpt || p->tab_cc != cc ||
+      p->tab_max != dpt_max) {
     p->tab = dedisp_tables(p->delays.data(), p->nchans, p->chans.data(), (int)p->chans.size(), first,
-                           count, dpt, cc);
+                           count, dpt, cc, dpt_max);
+    p->tab_max = dpt_max;
     p->tab_first = first;
     p->tab_count = count;
     p->tab_dpt = dpt;
@@ -188,8 +191,8 @@ const DedispTables &plan_host_tables(hdd_plan p, int first, int count, int dpt, 
   return p->tab;
 }
 
-hdd_error plan_device_tables(hdd_plan p, int first, int count, DeviceTables *out, int dpt, int cc) {
-  const DedispTables &t = plan_host_tables(p, first, count, dpt, cc);
+hdd_error plan_device_tables(hdd_plan p, int first, int count, DeviceTables *out, int dpt, int cc, int dpt_max) {
+  const DedispTables &t = plan_host_tables(p, first, count, dpt, cc, dpt_max);
   if (!p->tab_on_device) {
     const size_t mb = std::max<size_t>(t.meta.size(), 1) * sizeof(int4);
     const size_t ob = std::max<size_t>(t.off.size(), 1) * sizeof(int);
@@ -646,7 +649,8 @@ hdd_error hdd_execute_guru(hdd_plan p, hdd_size nsamps, const hdd_byte *in, hdd_
   const bool device = (flags & HDD_DEVICE_POINTERS) != 0;
 
   hg::DeviceTables tb;
-  hdd_error e = hg::plan_device_tables(p, (int)first_dm_idx, (int)dm_count, &tb);
+  hdd_error e = hg::plan_device_tables(p, (int)first_dm_idx, (int)dm_count, &tb, 0, 8,
+                                       hg::dedisp_tile_cap((int)dm_count, hg::dedisp_time_tiles(nout), 4));
   if (e != HDD_NO_ERROR) return e;
   const uint8_t *din = in;
   const size_t in_bytes = (size_t)(nsamps - 1) * in_stride + p->nchans;

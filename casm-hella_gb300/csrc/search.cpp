@@ -281,7 +281,8 @@ hella_status dedisperse_beam(hella_ctx *c, int beam, const hella_tuning &t) {
     return HELLA_OK;
   }
   hg::DeviceTables tb;
-  if (hg::plan_device_tables(c->plan, 0, c->ndms, &tb, t.dm_per_block, t.chan_chunk) != HDD_NO_ERROR)
+  const int cap = hg::dedisp_tile_cap(c->ndms, hg::dedisp_time_tiles(c->ntime_dd), t.add_mode ? 8 : 4);
+  if (hg::plan_device_tables(c->plan, 0, c->ndms, &tb, t.dm_per_block, t.chan_chunk, cap) != HDD_NO_ERROR)
     return HELLA_ERR_DEDISP;
   if (t.add_mode && tb.dpt < 8) return HELLA_ERR_INVALID_ARG;
   hg::DedispArgs a = hg::single_beam_args(tb, c->d_packed + (size_t)beam * c->p.nchan * c->R, c->R,
