@@ -89,6 +89,10 @@ cudaError_t pack_ring(const uint8_t *plain, uint32_t *packed, int nbeam,
 cudaError_t pack_gulp_dev(const uint8_t *plain, uint32_t *packed, int nbeam, int nchan,
                           long R, int gulp, const struct GulpPos *pos, cudaStream_t s,
                           const uint8_t *keep);
+// Packed words [nchan][R] of time-major input [nsamps][in_stride] (samples
+// past nsamps are zeros).
+cudaError_t pack_tf(const uint8_t *in, size_t in_stride, int nsamps, int nchan, uint32_t *packed, long R,
+                    cudaStream_t s);
 // Time-major input [nsamps][in_stride] -> channel-major plain [nchan][R].
 cudaError_t transpose_tf(const uint8_t *in, size_t in_stride, int nsamps,
                          int nchan, uint8_t *plain, long R, cudaStream_t s);

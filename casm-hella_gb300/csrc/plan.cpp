@@ -90,9 +90,9 @@ struct hdd_plan_struct {
   int4 *d_meta = nullptr;
   int *d_off = nullptr;
   size_t meta_cap = 0, off_cap = 0;
-  uint8_t *d_in = nullptr, *d_plain = nullptr, *d_out = nullptr;
+  uint8_t *d_in = nullptr, *d_out = nullptr;
   uint32_t *d_packed = nullptr;
-  size_t in_cap = 0, plain_cap = 0, out_cap = 0, packed_cap = 0;
+  size_t in_cap = 0, out_cap = 0, packed_cap = 0;
   // add-mode-4 tables of the last DM range used, host and device
   hg::SubTables sub;
   int sub_first = -1, sub_count = -1;
@@ -482,7 +482,6 @@ void hdd_destroy_plan(hdd_plan p) {
   cudaFree(p->d_off);
   cudaFree(p->d_err);
   cudaFree(p->d_in);
-  cudaFree(p->d_plain);
   cudaFree(p->d_packed);
   cudaFree(p->d_out);
   cudaFree(p->d_smeta);
@@ -661,8 +660,6 @@ hdd_error hdd_execute_guru(hdd_plan p, hdd_size nsamps, const hdd_byte *in, hdd_
     din = p->d_in;
   }
   const long R = ((long)nsamps + 3) / 4 * 4;
-  if ((e = grow((void **)&p->d_plain, &p->plain_cap, (size_t)p->nchans * R)) != HDD_NO_ERROR)
-    return e;
   if ((e = grow((void **)&p->d_packed, &p->packed_cap, (size_t)p->nchans * R * 4)) != HDD_NO_ERROR)
     return e;
   float *dout = reinterpret_cast<float *>(out);
@@ -671,10 +668,7 @@ hdd_error hdd_execute_guru(hdd_plan p, hdd_size nsamps, const hdd_byte *in, hdd_
       return e;
     dout = reinterpret_cast<float *>(p->d_out);
   }
-  if (hg::transpose_tf(din, in_stride, (int)nsamps, p->nchans, p->d_plain, R, p->stream) !=
-      cudaSuccess)
-    return HDD_INTERNAL_GPU_ERROR;
-  if (hg::pack_ring(p->d_plain, p->d_packed, 1, p->nchans, R, 0, R, p->stream) != cudaSuccess)
+  if (hg::pack_tf(din, in_stride, (int)nsamps, p->nchans, p->d_packed, R, p->stream) != cudaSuccess)
     return HDD_INTERNAL_GPU_ERROR;
   if (!p->d_err) {
     if (cudaMalloc((void **)&p->d_err, sizeof(int)) != cudaSuccess) {
@@ -718,9 +712,9 @@ hdd_error hdd_execute_guru(hdd_plan p, hdd_size nsamps, const hdd_byte *in, hdd_
       return HDD_MEM_COPY_FAILED;
   }
   if (!(flags & HDD_ASYNC)) {
-    if (cudaStreamSynchronize(p->stream) != cudaSuccess) return HDD_INTERNAL_GPU_ERROR;
-    int err = 0;
-    if (cudaMemcpy(&err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+    int err = 0;  // the status word follows the call's work on its stream: one wait for both
+    if (cudaMemcpyAsync(&err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost, p->stream) != cudaSuccess ||
+        cudaStreamSynchronize(p->stream) != cudaSuccess)
       return HDD_INTERNAL_GPU_ERROR;
     if (err) {
       cudaMemset(p->d_err, 0, sizeof(int));
