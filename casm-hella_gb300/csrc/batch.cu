@@ -893,10 +893,11 @@ hella_status hella_batch_create(hella_batch **out, const hella_batch_params *bp)
   DA(f.rowval, (size_t)nb * nch * 4);
   DA(f.scal, (size_t)nb * 8 * 4);
   DA(f.hsc, (size_t)nb * 8 * 2);
-  DA(f.lut, (size_t)nb * nch * 256 * 2);
+  DA(f.lut, (size_t)nb * hg::lut_slices(nch) * hg::kLutSl * 256 * 2);
   DA(f.flag2, (size_t)nb * nch);
   DA(f.ts, (size_t)nb * p->gulp * 4);
   DA(f.hts, (size_t)nb * p->gulp * 2);
+  DA(f.tdiv, (size_t)nb * p->gulp * 8);
   hg::flag_scrunch_params(*p, &f);
   if (p->nscrunch > 0 || f.f16_input) {
     DA(f.P, (size_t)nb * nch * p->gulp * 2);

@@ -33,160 +33,324 @@ namespace {
 __device__ __forceinline__ __half hzero() { return __float2half_rn(0.f); }
 __device__ __forceinline__ __half hone() { return __float2half_rn(1.f); }
 
-// Value of u8 level v of (beam b, channel c) after flagger stage `stage`:
+// Value of u8 level v of a channel after flagger stage `stage`:
 //  1 bandpass_correct   divide_by_bp (flagger.cu:180-194)
 //  2 normalize_data     (x + half(-mean)) * half(1/std) (flagger.cu:198-214)
 //  3 spectral flag      1, or x + 1 (replace_data_and_add_bandpass :146-158)
 //  4 bandpass_correct   of the final scrunch
-__device__ __half chain_value(int stage, int v, const FlagState &st, int b,
-                              int c) {
-  const int bc = b * st.nchan + c;
+struct ChanState {
+  float bp1, bp3;
+  bool flag2;
+  __half add, mul;
+};
+__device__ __half chain_value(int stage, int v, const ChanState &ch) {
   __half x = __float2half_rn((float)v);
-  if (stage >= 1) {
-    float bp = st.bp1[bc];
-    x = bp > 0.f ? __hdiv(x, __float2half_rn(bp)) : hzero();
-  }
-  if (stage >= 2) x = __hmul(__hadd(x, st.hsc[b * 8 + 0]), st.hsc[b * 8 + 1]);
-  if (stage >= 3) x = st.flag2[bc] ? hone() : __hadd(x, hone());
-  if (stage >= 4) {
-    float bp = st.bp3[bc];
-    x = bp > 0.f ? __hdiv(x, __float2half_rn(bp)) : hzero();
-  }
+  if (stage >= 1) x = ch.bp1 > 0.f ? __hdiv(x, __float2half_rn(ch.bp1)) : hzero();
+  if (stage >= 2) x = __hmul(__hadd(x, ch.add), ch.mul);
+  if (stage >= 3) x = ch.flag2 ? hone() : __hadd(x, hone());
+  if (stage >= 4) x = ch.bp3 > 0.f ? __hdiv(x, __float2half_rn(ch.bp3)) : hzero();
   return x;
 }
 
-__global__ void k_build_lut(FlagState st, int stage) {
-  const int c = blockIdx.x, b = blockIdx.y, v = threadIdx.x;
-  st.lut[((size_t)b * st.nchan + c) * 256 + v] = chain_value(stage, v, st, b, c);
+// The tables lie in slices of kLutSl channels, [level][channel]: a level's row
+// is whole words of channel pairs, and blocks stage rows or parts of them as
+// they are.  The last slice of a beam may be part empty.
+__device__ __forceinline__ __half *lut_row(__half *lut, int nchan, int b, int c, int level) {
+  return lut + (((size_t)b * ((nchan + kLutSl - 1) / kLutSl) + c / kLutSl) * 256 + level) * kLutSl + c % kLutSl;
 }
 
-// The row-statistics pass in a four-channel form: lane t of a warp holds
-// channels c0 + 4t .. c0 + 4t + 3 (one 32-bit load per row feeds four
-// chains, each summed in the reference's order), warps hold columns.  The
-// block's 128-channel slice of the table is staged as
-// lut_s[level * kQC + channel] through 16-byte loads of eight levels.
-constexpr int kQC = 128;
-constexpr int kRowT = 512;  // threads per block
-constexpr size_t kLutSlice = (size_t)256 * kQC * sizeof(__half);
-
-// Stages the table slice of channels c0 .. c0 + NC - 1 of beam b as
-// lut_s[level * NC + channel] (channels past nchan are left alone): each
-// thread loads eight levels of one channel with a 16-byte load, and the
-// lanes of a warp, holding consecutive channels, store without conflicts.
-template <int NC>
-__device__ __forceinline__ void load_lut_slice(__half *lut_s, const __half *lut, int nchan, int b, int c0) {
-  const int ncl = min(NC, nchan - c0);
-  const __half *lb = lut + ((size_t)b * nchan + c0) * 256;
-  for (int i = threadIdx.x; i < NC * 32; i += blockDim.x) {
-    const int cc = i % NC, vb = i / NC;  // levels 8vb .. 8vb+7 of channel cc
-    if (cc < ncl) {
-      const uint4 q = *reinterpret_cast<const uint4 *>(lb + (size_t)cc * 256 + 8 * vb);
-      const __half *h = reinterpret_cast<const __half *>(&q);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) lut_s[(8 * vb + k) * NC + cc] = h[k];
-    }
+// Warp tree over the 32 lane partials of a channel, / w (flagger.cu:103-111);
+// lane 0 has the result.
+__device__ __forceinline__ float lane_total(const float *part, int gulp) {
+  float v = part[threadIdx.x & 31];
+  for (int off = 16; off > 0; off /= 2) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
+  return __fdiv_rn(v, (float)gulp);
+}
+// Where that total goes.  mode 0: bp1, 1: bp2 + spectral flag, 2: bp3, 3: bpx.
+__device__ __forceinline__ void put_bandpass(const FlagState &st, int mode, int bc, float bp) {
+  if (mode == 0) st.bp1[bc] = bp;
+  if (mode == 1) {
+    st.bp2[bc] = bp;
+    st.flag2[bc] = (bp < st.spec_min || bp > st.spec_max) ? 1 : 0;
   }
+  if (mode == 2) st.bp3[bc] = bp;
+  if (mode == 3) st.bpx[bc] = bp;
 }
 
-// calc_bandpass_new partials: lane l of channel c sums samples l, l+32, ...
-// (below 32*floor(w/32)) in time order.  Block = 32 channels x 8 lanes, one
-// chain a thread (65536 chains for 2048 channels: too few for the
-// four-channel form to hide the memory latency); the row bytes are loaded
-// kLaneB at a time so that as many loads are in flight (64 a thread, about
-// 4 MB over the GPU; the two-blocks bound lets the compiler give them the
-// registers, 96, where it would otherwise fit 32 and interleave them with
-// the sums).  The table slice is staged as lut_s[level][channel] through
-// 16-byte loads of eight levels.
-constexpr int kLaneC = 32, kLaneB = 64;
-__global__ void __launch_bounds__(256, 2) k_lane_partials(const uint8_t *__restrict__ gulp,
-                                                       const __half *__restrict__ lut,
-                                                       float *__restrict__ part, int nchan, int w) {
-  __shared__ __half lut_s[256][kLaneC];
-  const int b = blockIdx.z, c0 = blockIdx.x * kLaneC;
-  load_lut_slice<kLaneC>(&lut_s[0][0], lut, nchan, b, c0);
-  __syncthreads();
-  const int cl = threadIdx.x & 31, l = blockIdx.y * 8 + (threadIdx.x >> 5);
-  const int c = c0 + cl;
-  const uint8_t *g = gulp + (size_t)b * w * nchan + (size_t)l * nchan + c;
-  const size_t step = (size_t)32 * nchan;
-  const int np = w / 32;
-  float s = 0.f;
-  int i = 0;
-  for (; i + kLaneB <= np; i += kLaneB) {
-    uint32_t v[kLaneB];
+// The tables of `stage`.  With fin >= 0 the lane partials of the pass before are
+// first brought to that mode's bandpass (a pass of its own would cost a launch,
+// 3 us, for 128 bytes a channel): every block does so for its own 32 channels, the
+// first of a column of blocks for all readers to come, and the values of its own
+// blocks come from shared memory.
+constexpr int kLutRows = 32, kLutC = 32;  // levels and channels a block
+__global__ void __launch_bounds__(256) k_build_lut(FlagState st, int stage, int fin) {
+  __shared__ float bp_s[kLutC];
+  const int cl = threadIdx.x % kLutC, c0 = blockIdx.x * kLutC, b = blockIdx.z, wi = threadIdx.x / 32;
+  const int bc0 = b * st.nchan + c0;
+  if (fin >= 0) {
 #pragma unroll
-    for (int u = 0; u < kLaneB; ++u) v[u] = g[(size_t)(i + u) * step];
-#pragma unroll
-    for (int u = 0; u < kLaneB; ++u) s = __fadd_rn(s, __half2float(lut_s[v[u]][cl]));
-  }
-  for (; i < np; ++i) s = __fadd_rn(s, __half2float(lut_s[g[(size_t)i * step]][cl]));
-  part[((size_t)b * nchan + c) * 32 + l] = s;
-}
-
-// computeRowMeans / computeRowVariances partials: column j of channel c
-// sums columns j, j+256, ... below nw = 256*floor(w/256).  TS: values
-// divided by half(ts[t]) (divide_by_ts, timeseries.cu:38-55).  VAR:
-// (x - mean)^2 with the fused multiply-add the reference's compiler emits.
-// The two-blocks bound gives the unrolled loads registers (44-64 instead of
-// 32), as in k_lane_partials.
-template <bool VAR, bool TS>
-__global__ void __launch_bounds__(kRowT, 2) k_row_partials(const uint8_t *__restrict__ gulp, FlagState st,
-                                                            int which) {
-  extern __shared__ __align__(16) __half lut4_s[];
-  const int b = blockIdx.z, c0 = blockIdx.x * kQC, nchan = st.nchan, w = st.gulp;
-  load_lut_slice<kQC>(lut4_s, st.lut, nchan, b, c0);
-  __syncthreads();
-  const int cq = 4 * (threadIdx.x & 31), c = c0 + cq;
-  const int j = blockIdx.y * (kRowT / 32) + (threadIdx.x >> 5);
-  if (c >= nchan) return;
-  const uint8_t *g = gulp + (size_t)b * w * nchan + (size_t)j * nchan + c;
-  const __half *hts = st.hts + (size_t)b * w + j;
-  const size_t step = (size_t)256 * nchan;
-  const int nk = w / 256;
-  const float mean = VAR ? st.scal[b * 8 + 2 * which] : 0.f;
-  const __half *ls = lut4_s + cq;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-  for (int k = 0; k < nk; ++k) {
-    const uint32_t x = *reinterpret_cast<const uint32_t *>(g + k * step);
-    __half th;
-    if (TS) th = hts[k * 256];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      __half hv = ls[((x >> (8 * q)) & 255u) * kQC + q];
-      if (TS) hv = __hdiv(hv, th);
-      const float f = __half2float(hv);
-      if (VAR) {
-        const float d = __fsub_rn(f, mean);
-        acc[q] = __fmaf_rn(d, d, acc[q]);
-      } else {
-        acc[q] = __fadd_rn(acc[q], f);
+    for (int i = wi; i < kLutC; i += 8) {
+      const float bp = lane_total(st.part + (size_t)(bc0 + i) * 32, st.gulp);
+      if (cl == 0) {
+        bp_s[i] = bp;
+        if (blockIdx.y == 0) put_bandpass(st, fin, bc0 + i, bp);
       }
     }
+    __syncthreads();
   }
-  float *pp = st.part + ((size_t)b * nchan + c) * 256 + j;
+  const int bc = bc0 + cl;
+  ChanState ch{};
+  if (stage >= 1) ch.bp1 = fin == 0 ? bp_s[cl] : st.bp1[bc];
+  if (stage >= 3) {
+    ch.flag2 = fin == 1 ? bp_s[cl] < st.spec_min || bp_s[cl] > st.spec_max : st.flag2[bc] != 0;
+  }
+  if (stage >= 4) ch.bp3 = fin == 2 ? bp_s[cl] : st.bp3[bc];
+  if (stage >= 2) {
+    ch.add = st.hsc[b * 8 + 0];
+    ch.mul = st.hsc[b * 8 + 1];
+  }
+  __half *row = lut_row(st.lut, st.nchan, b, c0 + cl, 0);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) pp[q * 256] = acc[q];
+  for (int v = blockIdx.y * kLutRows + wi, i = 0; i < kLutRows / 8; ++i, v += 8)
+    row[v * kLutSl] = chain_value(stage, v, ch);
 }
 
-// Warp tree over the 32 lane partials, / w (flagger.cu:103-111).  One warp
-// per (beam, channel).  mode 0: bp1, 1: bp2 + spectral flag, 2: bp3.
+// Stages the table of channels c0 .. c0 + NC - 1 of beam b (within one slice) as
+// lut_s[level * NC + channel] with 16-byte loads of eight channels of a level;
+// channels past the slice's last hold anything.
+template <int NC>
+__device__ __forceinline__ void load_lut_slice(__half *lut_s, __half *lut, int nchan, int b, int c0) {
+  const __half *src = lut_row(lut, nchan, b, c0, 0);
+  for (int i = threadIdx.x; i < NC * 32; i += blockDim.x) {
+    const int v = i / (NC / 8), k = 8 * (i % (NC / 8));
+    *reinterpret_cast<uint4 *>(lut_s + v * NC + k) = *reinterpret_cast<const uint4 *>(src + v * kLutSl + k);
+  }
+}
+
+// a / b for half-precision a, b with r = 1 / b rounded: one correction step
+// after a first product (P. Markstein, IBM J. Res. Dev. 34, 1990) gives the
+// float quotient, whose rounding to half is the half quotient (24 bits are twice
+// 11 and two more).  Not for zero, infinite or NaN b, nor for such a quotient: the
+// correction then makes NaN or infinity of them, which callers look for and
+// leave to __hdiv.  (A zero of the other sign may come out for -0 / b.)
+__device__ __forceinline__ float div_step(float a, float b, float r) {
+  const float q = __fmul_rn(a, r);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
+// The sums over time.  MOD = 32, calc_bandpass_new: lane l of channel c sums
+// samples l, l + 32, ... (below 32 floor(w / 32)) in time order.  MOD = 256,
+// computeRowMeans / computeRowVariances: column j sums samples j, j + 256, ...
+// below 256 floor(w / 256).  RAW: the levels themselves; else their table values.
+// TS: values divided by half(ts[t]) (divide_by_ts, timeseries.cu:38-55).  VAR:
+// (x - mean)^2 with the fused multiply-add the reference's compiler emits.
+//
+// A warp takes 32 CH channels of one sum after another (`per` of them), a lane CH
+// neighbouring ones: one load a row feeds CH sums.  The block's table slice is in
+// shared memory as it lies in global memory, [level][pair]; with CH = 4 the upper
+// 16 lanes take their channel pairs in the other order, so that a lookup of a
+// warp never hits a bank twice, and one byte permute makes the address from level
+// and lane.  Each warp's rows (and their divisors) arrive by asynchronous copies,
+// ROWS a stage, AHEAD stages on their way, without block-wide waits.  Raw levels
+// are added two to a word, a stage at a time: whole numbers below 2^24, the same
+// in any order (kRawMax).  Bound by instruction issue and the lookups (shared
+// memory): 8 beams x 32,768 samples x 1024 channels 65 us (94 us with a
+// half-precision lookup on two banks and eight rows in flight a thread), divided
+// by ts 104 us (146 us), lane sums 58 us (117 us), of levels 41 us.
+constexpr int kSumWarps = 8;
+constexpr int kLutBytes = kLutSl * 256 * (int)sizeof(__half);
+constexpr int kRawMax = (1 << 24) / 255;  // levels that a float adds up exactly
+constexpr int sum_stage(int rows, int ch, bool ts) { return rows * (32 * ch + (ts ? 8 : 0)); }  // bytes
+template <int N>
+__device__ __forceinline__ void copy_async(void *d, const void *src) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(d);
+  if (N == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(src) : "memory");
+}
+template <int MOD, bool VAR, bool TS, bool RAW, int CH, int ROWS, int AHEAD>
+__global__ void __launch_bounds__(32 * kSumWarps, 2) k_sums(const uint8_t *__restrict__ gulp, FlagState st, int which,
+                                                            int per) {
+  extern __shared__ __align__(16) uint8_t sum_s[];
+  constexpr int kRowB = 32 * CH, kPieces = kRowB / 16, kStep = 32 / kPieces;  // bytes and 16-byte pieces of a row; rows a copy
+  constexpr int kDepth = AHEAD + 1, kStage = ROWS * (kRowB + (TS ? 8 : 0));
+  const int b = blockIdx.z, c0 = blockIdx.x * kLutSl, nchan = st.nchan, w = st.gulp;
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  constexpr int kParts = 4 / CH;  // warps side by side on the slice
+  const int part = wi % kParts, cw = c0 + part * kRowB, nw = (blockDim.x >> 5) / kParts;
+  if (!RAW) {
+    const uint8_t *src = reinterpret_cast<const uint8_t *>(lut_row(st.lut, nchan, b, c0, 0));
+#pragma unroll 4
+    for (int i = threadIdx.x * 16; i < kLutBytes; i += blockDim.x * 16) copy_async<16>(sum_s + i, src + i);
+  }
+  uint8_t *ring = sum_s + (RAW ? 0 : kLutBytes) + wi * kDepth * kStage;
+  const int nk = w / MOD, nst = (nk + ROWS - 1) / ROWS;
+  const int j0 = blockIdx.y * per * nw + wi / kParts, total = per * nst;
+  // the copies: this lane's place in a stage, the row it reads next and its sum
+  const int pr = lane / kPieces, pk = lane % kPieces;
+  const size_t step = (size_t)MOD * nchan;
+  const bool piece = cw + 16 * pk < nchan;
+  const uint8_t *const first_row = gulp + (size_t)b * w * nchan + cw + 16 * pk + pr * step;
+  const uint8_t *src = first_row + (size_t)j0 * nchan;
+  const float2 *tsrc = TS ? st.tdiv + (size_t)b * w + j0 + lane * MOD : nullptr;
+  int lj = j0, lk = 0, lslot = 0, left = total;
+  auto load = [&]() {
+    if (left > 0) {
+      uint8_t *d = ring + lslot + pr * kRowB + 16 * pk;
+#pragma unroll
+      for (int u = 0; u < ROWS; u += kStep)
+        if (piece && lk + u + pr < nk) copy_async<16>(d + u * kRowB, src + u * step);
+      if (TS && lane < ROWS && lk + lane < nk) copy_async<8>(ring + lslot + ROWS * kRowB + lane * 8, tsrc);
+      --left;
+      lslot = lslot == AHEAD * kStage ? 0 : lslot + kStage;
+      lk += ROWS;
+      src += ROWS * step;
+      if (TS) tsrc += ROWS * MOD;
+      if (lk >= nk) {
+        lk = 0;
+        lj += nw;
+        src = first_row + (size_t)lj * nchan;
+        if (TS) tsrc = st.tdiv + (size_t)b * w + lj + lane * MOD;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const float mean = VAR ? st.scal[b * 8 + 2 * which] : 0.f;
+#pragma unroll 1
+  for (int i = 0; i < AHEAD; ++i) load();
+  const bool hi = CH == 4 && lane >= 16;
+  // addresses of channels 0, 1 and (CH = 4) 2, 3 as taken, without the level
+  const uint32_t first = 128u * part + 2u * CH * lane + (hi ? 4u : 0u);
+  const uint32_t second = 8u * lane + (hi ? 0u : 4u);
+  const bool exact = RAW && nk <= kRawMax;
+  float acc[CH];
+  uint32_t total_s[CH];
+#pragma unroll
+  for (int q = 0; q < CH; ++q) acc[q] = 0.f, total_s[q] = 0u;
+  if (!RAW) {  // the whole table, from all threads
+    asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
+    __syncthreads();
+  }
+  // one row; `fast`: quotients by div_step, else by __hdiv
+  auto row = [&](const uint8_t *d, int r, bool fast) {
+    uint32_t x;
+    if (CH == 4) {
+      x = *reinterpret_cast<const uint32_t *>(d + r * kRowB + 4 * lane);
+      x = __byte_perm(x, x, hi ? 0x1032 : 0x3210);
+    } else {
+      x = *reinterpret_cast<const uint16_t *>(d + r * kRowB + 2 * lane);
+    }
+    float f[CH];
+    if (RAW) {
+#pragma unroll
+      for (int q = 0; q < CH; ++q)
+        f[q] = __fsub_rn(__uint_as_float(__byte_perm(x, 0x4b000000u, 0x7440 + q)), 8388608.f);  // 2^23 + level - 2^23
+    } else {
+      __half h[CH];
+#pragma unroll
+      for (int q = 0; q < CH; ++q)
+        h[q] = *reinterpret_cast<const __half *>(sum_s + __byte_perm(x, q < 2 ? first : second, 0x7704 + 16 * q) +
+                                                 2 * (q & 1));
+#pragma unroll
+      for (int q = 0; q < CH; ++q) f[q] = __half2float(h[q]);
+      if (TS) {
+        const float2 t = *reinterpret_cast<const float2 *>(d + ROWS * kRowB + r * 8);
+        if (fast) {
+#pragma unroll
+          for (int q = 0; q < CH; q += 2) {
+            const __half2 p = __floats2half2_rn(div_step(f[q], t.x, t.y), div_step(f[q + 1], t.x, t.y));
+            f[q] = __low2float(p);
+            f[q + 1] = __high2float(p);
+          }
+        } else {
+          const __half th = __float2half_rn(t.x);
+#pragma unroll
+          for (int q = 0; q < CH; ++q) f[q] = __half2float(__hdiv(h[q], th));
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < CH; ++q) {
+      if (VAR) {
+        const float e = __fsub_rn(f[q], mean);
+        acc[q] = __fmaf_rn(e, e, acc[q]);
+      } else {
+        acc[q] = __fadd_rn(acc[q], f[q]);
+      }
+    }
+  };
+  int slot = 0, k0 = 0, j = j0;
+#pragma unroll 1
+  for (int i = 0; i < total; ++i) {
+    load();  // its slot was read in the iteration before, behind __syncwarp
+    asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
+    __syncwarp();
+    const uint8_t *d = ring + slot;
+    slot = slot == AHEAD * kStage ? 0 : slot + kStage;
+    const int n = min(ROWS, nk - k0);
+    if (RAW && exact) {
+      uint32_t even = 0u, odd = 0u;  // sums of bytes 0, 2 and 1, 3: at most 255 ROWS each
+      static_assert(ROWS <= 256, "16 bits a sum");
+#pragma unroll 8
+      for (int r = 0; r < n; ++r) {
+        const uint32_t x = *reinterpret_cast<const uint32_t *>(d + r * kRowB + 4 * lane);
+        even += x & 0x00ff00ffu;
+        odd += (x >> 8) & 0x00ff00ffu;
+      }
+      total_s[0] += even & 0xffffu;
+      total_s[1] += odd & 0xffffu;
+      total_s[CH - 2] += even >> 16;
+      total_s[CH - 1] += odd >> 16;
+    } else {
+      float before[CH];
+#pragma unroll
+      for (int q = 0; q < CH; ++q) before[q] = acc[q];
+      if (n == ROWS) {
+#pragma unroll 8
+        for (int r = 0; r < ROWS; ++r) row(d, r, true);
+      } else {
+#pragma unroll 1
+        for (int r = 0; r < n; ++r) row(d, r, true);
+      }
+      if (TS) {  // a quotient that div_step does not give leaves its sum infinite or NaN
+        bool finite = true;
+#pragma unroll
+        for (int q = 0; q < CH; ++q) finite = finite && fabsf(acc[q]) <= 3.0e38f;
+        if (!finite) {
+#pragma unroll
+          for (int q = 0; q < CH; ++q) acc[q] = before[q];
+#pragma unroll 1
+          for (int r = 0; r < n; ++r) row(d, r, false);
+        }
+      }
+    }
+    k0 += ROWS;
+    if (k0 >= nk) {
+      const int c = cw + CH * lane;
+      float *pp = st.part + ((size_t)b * nchan + c) * MOD + j;
+      if (c < nchan)
+#pragma unroll
+        for (int q = 0; q < CH; ++q)
+          if (RAW && exact)
+            pp[q * MOD] = (float)total_s[q];
+          else
+            pp[(hi ? q ^ 2 : q) * MOD] = acc[q];
+#pragma unroll
+      for (int q = 0; q < CH; ++q) acc[q] = 0.f, total_s[q] = 0u;
+      k0 = 0;
+      j += nw;
+    }
+    __syncwarp();
+  }
+}
+
+// lane_total by itself, one warp per (beam, channel).
 __global__ void k_lane_finish(FlagState st, int mode) {
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
   if (gw >= st.nbeam * st.nchan) return;
-  float v = st.part[(size_t)gw * 32 + lane];
-  for (int off = 16; off > 0; off /= 2) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
-  if (lane == 0) {
-    float bp = __fdiv_rn(v, (float)st.gulp);
-    if (mode == 0) st.bp1[gw] = bp;
-    if (mode == 1) {
-      st.bp2[gw] = bp;
-      st.flag2[gw] = (bp < st.spec_min || bp > st.spec_max) ? 1 : 0;
-    }
-    if (mode == 2) st.bp3[gw] = bp;
-    if (mode == 3) st.bpx[gw] = bp;
-  }
+  const float bp = lane_total(st.part + (size_t)gw * 32, st.gulp);
+  if ((threadIdx.x & 31) == 0) put_bandpass(st, mode, gw, bp);
 }
 
 // Thread 0 of the reference's 256-thread block: each warp's shuffle tree,
@@ -273,41 +437,151 @@ unsigned lane_finish(const FlagState &st, int mode, int fin_blocks, cudaStream_t
 }
 
 // measure_ts: per sample, fp16 running sum over channels in channel order,
-// then ts = float(sum) / nchan.  Block = 128 consecutive samples; rows and
-// table slices are staged through shared memory 64 channels at a time.
-// The gulp rows and table slices are staged with 4- and 16-byte loads
-// (nchan % 32 == 0 keeps every 64-channel chunk whole and aligned).
-constexpr int kTsT = 128, kTsC = 64;
-__global__ void __launch_bounds__(kTsT) k_ts(const uint8_t *__restrict__ gulp,
-                                             FlagState st) {
-  __shared__ __align__(16) uint8_t rows_s[kTsT][kTsC + 4];
-  __shared__ __align__(16) __half lut_s[kTsC][256];
-  const int b = blockIdx.y, t0 = blockIdx.x * kTsT, nchan = st.nchan, w = st.gulp;
-  const int tid = threadIdx.x;
-  const uint8_t *g = gulp + (size_t)b * w * nchan + (size_t)t0 * nchan;
-  const __half *lb = st.lut + (size_t)b * nchan * 256;
-  __half s = hzero();
-  for (int c0 = 0; c0 < nchan; c0 += kTsC) {
-    const int nc = min(kTsC, nchan - c0);
-    __syncthreads();
-    for (int i = tid; i < kTsT * (kTsC / 4); i += kTsT) {
-      const int r = i / (kTsC / 4), c4 = 4 * (i % (kTsC / 4));
-      if (c4 < nc && t0 + r < w)
-        *reinterpret_cast<uint32_t *>(&rows_s[r][c4]) =
-            *reinterpret_cast<const uint32_t *>(g + (size_t)r * nchan + c0 + c4);
+// then ts = float(sum) / nchan.  A lane holds a sample; lane l is l channel
+// pairs behind lane 0, so the 32 lanes of a warp look up 32 different pairs,
+// and with the table as [level][pair] every lookup of a warp hits 32 different
+// banks whatever the levels are (with all lanes on one channel the levels fall
+// on random banks, three to four passes a lookup).  An iteration takes two
+// pairs of every lane; the first and last 16 leave out what lies outside.
+// The table (kTsSlots chunks of kTsC channels, two 64 KB halves of 64 pairs: a
+// byte permute puts level, pair and half into an address) and each warp's 32
+// gulp rows (kTsRows chunks) are rings that asynchronous copies fill one chunk
+// ahead.  Bound by the lookups (shared memory): 65,536 samples x 2048 channels
+// 48 us, 147 us with the lanes on one channel.
+constexpr int kTsC = 64, kTsSlots = 4, kTsRows = 3;
+constexpr int kTsLut = kTsSlots * kTsC * 256 * (int)sizeof(__half);  // bytes of the table ring
+constexpr int kTsPitch = kTsRows * kTsC;                            // bytes of a ring row: even lanes' words and
+                                                                    // odd lanes' fall on different banks
+constexpr int kTsWarps = 16;                                        // most sums a block (warps)
+__host__ __device__ constexpr int ts_smem(int nw) { return kTsLut + nw * 32 * kTsPitch; }
+__global__ void __launch_bounds__(32 * kTsWarps) k_ts(const uint8_t *__restrict__ gulp, FlagState st, int nw) {
+  extern __shared__ __align__(16) uint8_t ts_s[];
+  const int b = blockIdx.y, nchan = st.nchan, w = st.gulp;
+  const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
+  const int t0 = (blockIdx.x * nw + wi) * 32;
+  const bool live = wi < nw && t0 < w;  // the other warps only copy (w % 32 == 0: whole warps)
+  uint8_t *rows = ts_s + kTsLut + wi * 32 * kTsPitch;
+  const uint8_t *g = gulp + ((size_t)b * w + t0) * nchan;
+  const int nchunk = (nchan + kTsC - 1) / kTsC;
+  auto copy16 = [](void *d, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src)
+                 : "memory");
+  };
+  // a thread's part of each chunk: table rows lv, lv + lstep, .., channels 8 lk .. + 7; gulp rows rr,
+  // rr + 8, .., bytes 16 rk .. + 15
+  constexpr int kLk = kTsC / 8, kRk = kTsC / 16;
+  const int lk = tid % kLk, lv = tid / kLk, lstep = blockDim.x / kLk, rk = lane % kRk, rr = lane / kRk;
+  auto load = [&](int m) {  // chunk m of the table and the rows
+    if (m < nchunk) {
+      uint8_t *d = ts_s + (m & 2) * (kTsLut / 4) + (m & 1) * (kTsC * 2) + lv * 256 + lk * 16;
+      const __half *src = lut_row(st.lut, nchan, b, m * kTsC, lv) + 8 * lk;
+#pragma unroll 4
+      for (int v = lv; v < 256; v += lstep, d += lstep * 256, src += lstep * kLutSl) copy16(d, src);
+      if (live && m * kTsC + rk * 16 < nchan) {
+        uint8_t *e = rows + rr * kTsPitch + m % kTsRows * kTsC + rk * 16;
+        const uint8_t *q = g + (size_t)rr * nchan + m * kTsC + rk * 16;
+#pragma unroll
+        for (int r = 0; r < 32; r += 32 / kRk) copy16(e + r * kTsPitch, q + (size_t)r * nchan);
+      }
     }
-    const uint4 *lsrc = reinterpret_cast<const uint4 *>(lb + (size_t)c0 * 256);
-    uint4 *ldst = reinterpret_cast<uint4 *>(&lut_s[0][0]);
-    for (int i = tid; i < nc * 256 / 8; i += kTsT) ldst[i] = lsrc[i];
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int nq = nchan / 4, np = nchan / 2;
+  const uint32_t sel = lane & 1 ? 0x5432u : 0x7654u;  // odd lanes start in the middle of a word of four channels
+  uint32_t y = (4u * (128u - lane)) & 0x1ffu;         // 4 x pair, modulo the table ring
+  uint32_t rq = (kTsPitch - 4 * (lane / 2)) % kTsPitch;  // byte in the ring row
+  uint32_t prev = 0;
+  __half s = hzero();
+  const uint8_t *rl = rows + lane * kTsPitch;
+  auto iterate = [&](int i, bool edge) {
+    const uint32_t cur = *reinterpret_cast<const uint32_t *>(rl + rq);
+    const uint32_t x = __byte_perm(prev, cur, sel), y1 = (y + 4u) & 0x1ffu;
+    prev = cur;
+    __half v[4];
+    v[0] = *reinterpret_cast<const __half *>(ts_s + __byte_perm(x, y, 0x7504));
+    v[1] = *reinterpret_cast<const __half *>(ts_s + __byte_perm(x, y, 0x7514) + 2);
+    v[2] = *reinterpret_cast<const __half *>(ts_s + __byte_perm(x, y1, 0x7524));
+    v[3] = *reinterpret_cast<const __half *>(ts_s + __byte_perm(x, y1, 0x7534) + 2);
+    if (edge) {  // adding +0 changes no sum: it starts at +0 and is never -0
+      const int p = 2 * i - lane;
+      if (p < 0 || p >= np) v[0] = v[1] = hzero();
+      if (p + 1 < 0 || p + 1 >= np) v[2] = v[3] = hzero();
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s = __hadd(s, v[k]);
+    y = (y + 8u) & 0x1ffu;
+    rq = min(rq + 4u, rq + 4u - (uint32_t)kTsPitch);
+  };
+  constexpr int kIt = kTsC / 4;  // iterations a chunk; 16 more after the last channel
+  load(0);
+  for (int m = 0; m * kIt < nq + 16; ++m) {
+    load(m + 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    if (t0 + tid < w)
-      for (int cc = 0; cc < nc; ++cc) s = __hadd(s, lut_s[cc][rows_s[tid][cc]]);
+    if (live) {
+      const int i0 = m * kIt, i1 = min(i0 + kIt, nq + 16);
+      if (i0 >= 16 && i1 <= nq) {
+#pragma unroll 8
+        for (int i = i0; i < i1; ++i) iterate(i, false);
+      } else {
+#pragma unroll 1
+        for (int i = i0; i < i1; ++i) iterate(i, true);
+      }
+    }
+    __syncthreads();  // chunk m - 1 is overwritten next
   }
-  if (t0 + tid < w) {
-    float ts = __fdiv_rn(__half2float(s), (float)nchan);
-    st.ts[(size_t)b * w + t0 + tid] = ts;
-    st.hts[(size_t)b * w + t0 + tid] = __float2half_rn(ts);
+  if (live) {
+    const float ts = __fdiv_rn(__half2float(s), (float)nchan);
+    st.ts[(size_t)b * w + t0 + lane] = ts;
+    const __half h = __float2half_rn(ts);
+    st.hts[(size_t)b * w + t0 + lane] = h;
+    st.tdiv[(size_t)b * w + t0 + lane] = make_float2(__half2float(h), __frcp_rn(__half2float(h)));
   }
+}
+
+// Launches k_sums.  Lane sums have 32 chains a channel: with fewer than four
+// warps an SM in all, a lane takes two channels (twice the warps; levels are added
+// two to a word anyway), blocks are as small as spreads them over the SMs and
+// 32-row stages keep their fixed cost down (512 channels x 16,384 samples: 10.7 us,
+// levels 9.1 us, 16 us with one chain a thread and 64 loads in flight); else, and for the row sums, 8 warps
+// a block, two blocks an SM.
+template <int MOD, bool VAR, bool TS, bool RAW, int CH, int ROWS, int AHEAD>
+cudaError_t launch_sums(const FlagState &st, const uint8_t *gulp, int which, int nw, int per, cudaStream_t s) {
+  const auto k = k_sums<MOD, VAR, TS, RAW, CH, ROWS, AHEAD>;
+  const int smem = (RAW ? 0 : kLutBytes) + nw * (AHEAD + 1) * sum_stage(ROWS, CH, TS);
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k<<<dim3(lut_slices(st.nchan), MOD / (nw * CH / 4 * per), st.nbeam), 32 * nw, smem, s>>>(gulp, st, which, per);
+  return cudaSuccess;
+}
+template <bool RAW>
+cudaError_t launch_lanes(const FlagState &st, const uint8_t *gulp, cudaStream_t s) {
+  const long warps = 32L * lut_slices(st.nchan) * st.nbeam;
+  if (warps > 4 * 152) return launch_sums<32, false, false, RAW, 4, 16, 2>(st, gulp, 0, kSumWarps, 1, s);
+  constexpr int kCh = RAW ? 4 : 2;
+  const int lanes = warps > 2 * 152 ? 4 : warps > 152 ? 2 : 1;  // a block
+  return launch_sums<32, false, false, RAW, kCh, 32, RAW ? 4 : 3>(st, gulp, 0, lanes * 4 / kCh, 1, s);
+}
+template <bool VAR, bool TS>
+cudaError_t launch_rows(const FlagState &st, const uint8_t *gulp, int which, cudaStream_t s) {
+  // several sums a warp where that leaves three blocks for each that fits: the table is staged less often
+  const long blocks = 256L / kSumWarps * lut_slices(st.nchan) * st.nbeam;
+  const int per = blocks >= 4 * 3 * 304 ? 4 : blocks >= 2 * 3 * 304 ? 2 : 1;
+  return launch_sums<256, VAR, TS, false, 4, 8, 4>(st, gulp, which, kSumWarps, per, s);
+}
+
+// Launches k_ts with as many warps a block as fill whole rounds of one block
+// an SM (the table ring leaves no room for two), and four at least to copy.
+cudaError_t launch_ts(const FlagState &st, const uint8_t *gulp, cudaStream_t s) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_ts, cudaFuncAttributeMaxDynamicSharedMemorySize, ts_smem(kTsWarps));
+  if (e != cudaSuccess) return e;
+  const long per = st.gulp / 32, warps = per * st.nbeam;
+  const long rounds = (warps + 152 * kTsWarps - 1) / (152 * kTsWarps);
+  const int nw = (int)((warps + 152 * rounds - 1) / (152 * rounds));
+  k_ts<<<dim3((unsigned)((per + nw - 1) / nw), st.nbeam), 32 * std::max(nw, 4), ts_smem(std::max(nw, 4)), s>>>(gulp, st,
+                                                                                                          nw);
+  return cudaSuccess;
 }
 
 // transpose_output (transpose.cu:321-331): u8 = trunc(clamp(255/14 (x+4))).
@@ -332,7 +606,7 @@ __global__ void __launch_bounds__(256) k_flag_out(const uint8_t *__restrict__ gu
                                                   uint8_t *__restrict__ plain, long R, long wpos,
                                                   const GulpPos *dpos) {
   if (dpos) wpos = dpos->wpos;
-  __shared__ __half lut_s[256][kOutC];
+  __shared__ __align__(16) __half lut_s[256][kOutC];
   __shared__ __align__(16) uint8_t tile[kOutC][kOutT + 4];
   const int b = blockIdx.z, c0 = blockIdx.x * kOutC, t0 = blockIdx.y * kOutT;
   const int nchan = st.nchan, w = st.gulp, tid = threadIdx.x;
@@ -377,11 +651,10 @@ __global__ void k_plane_init(const uint8_t *__restrict__ gulp, FlagState st) {
 #pragma unroll
   for (int j = 0; j < 32; j += 8) tile[ty + j][tx] = g[(size_t)(t0 + ty + j) * nchan + c0 + tx];
   __syncthreads();
-  const __half *lb = st.lut + (size_t)b * nchan * 256;
 #pragma unroll
   for (int j = 0; j < 32; j += 8) {
     const int c = c0 + ty + j;
-    st.P[((size_t)b * nchan + c) * w + t0 + tx] = lb[(size_t)c * 256 + tile[tx][ty + j]];
+    st.P[((size_t)b * nchan + c) * w + t0 + tx] = *lut_row(st.lut, nchan, b, c, tile[tx][ty + j]);
   }
 }
 
@@ -565,7 +838,6 @@ namespace {
 // from the data after bandpass_flag.
 cudaError_t scrunch_planes(const FlagState &st, const void *gulp, uint8_t *plain, long R, long wpos,
                            const GulpPos *dpos, cudaStream_t s) {
-  const dim3 lutg(st.nchan, st.nbeam);
   const int fin_blocks = (st.nbeam * st.nchan * 32 + 255) / 256;
   const size_t n = (size_t)st.nbeam * st.nchan * st.gulp;
   const int eb = (int)std::min<size_t>((n + 255) / 256, 152 * 16);
@@ -598,10 +870,9 @@ cudaError_t scrunch_planes(const FlagState &st, const void *gulp, uint8_t *plain
     k_plane_spec<<<eb, 256, 0, s>>>(st);
     launches += 3;
   } else {
-    k_build_lut<<<lutg, 256, 0, s>>>(st, 3);
     k_plane_init<<<dim3(st.nchan / 32, st.gulp / 32, st.nbeam), dim3(32, 8), 0, s>>>(
         static_cast<const uint8_t *>(gulp), st);
-    launches += 2;
+    launches += 1;
   }
   for (int e = 0; e < st.nscrunch; ++e) {
     const int xw = st.sc_t[e], yw = st.sc_f[e];
@@ -638,60 +909,54 @@ cudaError_t flag_impl(const FlagState &st, const void *gulp_in, uint8_t *plain, 
                       const GulpPos *dpos, cudaStream_t s) {
   if (st.f16_input) return scrunch_planes(st, gulp_in, plain, R, wpos, dpos, s);
   const uint8_t *gulp = static_cast<const uint8_t *>(gulp_in);
-  const dim3 lutg(st.nchan, st.nbeam);
-  const dim3 laneg(st.nchan / kLaneC, 32 / 8, st.nbeam);
-  const dim3 rowg((st.nchan + kQC - 1) / kQC, 256 / (kRowT / 32), st.nbeam);
-  {  // the table slice is above the default 48 KB of dynamic shared memory
-    const int lb = (int)kLutSlice;
-    cudaError_t e = cudaFuncSetAttribute(k_row_partials<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_row_partials<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_row_partials<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_row_partials<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
-    if (e != cudaSuccess) return e;
-  }
+  const dim3 lutg(st.nchan / kLutC, 256 / kLutRows, st.nbeam);
   const int fin_blocks = (st.nbeam * st.nchan * 32 + 255) / 256;
 
-  // bandpass_flag: bandpass_correct (calc_bandpass_new, divide_by_bp)
-  k_build_lut<<<lutg, 256, 0, s>>>(st, 0);
-  k_lane_partials<<<laneg, 256, 0, s>>>(gulp, st.lut, st.part, st.nchan, st.gulp);
-  unsigned extra = lane_finish(st, 0, fin_blocks, s) - 1;
-  k_build_lut<<<lutg, 256, 0, s>>>(st, 1);
-  // normalize_data: calculate_stddev (mean pass, variance pass)
-  k_row_partials<false, false><<<rowg, kRowT, kLutSlice, s>>>(gulp, st, 0);
-  k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-  k_beam_sum<false><<<st.nbeam, kBeamT, 0, s>>>(st, 0);
-  k_row_partials<true, false><<<rowg, kRowT, kLutSlice, s>>>(gulp, st, 0);
-  k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-  k_beam_sum<true><<<st.nbeam, kBeamT, 0, s>>>(st, 0);
+  cudaError_t e = cudaSuccess;
+  unsigned launches = 0;
+  // lane sums, the bandpass of `mode` and the tables of `stage` with it (through the
+  // median filter where bandpass_correct applies it)
+  auto bandpass = [&](bool raw, int mode, int stage) {
+    if (e == cudaSuccess) e = raw ? launch_lanes<true>(st, gulp, s) : launch_lanes<false>(st, gulp, s);
+    ++launches;
+    const bool median = mode != 1 && st.bp_median > 1;
+    if (median) launches += lane_finish(st, mode, fin_blocks, s);
+    if (stage >= 0) {
+      k_build_lut<<<lutg, 256, 0, s>>>(st, stage, median ? -1 : mode);
+      ++launches;
+    } else if (!median) {
+      launches += lane_finish(st, mode, fin_blocks, s);
+    }
+  };
+  auto normalize = [&](int which) {  // calculate_stddev: mean pass, variance pass
+    if (e == cudaSuccess) e = which ? launch_rows<false, true>(st, gulp, which, s) : launch_rows<false, false>(st, gulp, which, s);
+    k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
+    k_beam_sum<false><<<st.nbeam, kBeamT, 0, s>>>(st, which);
+    if (e == cudaSuccess) e = which ? launch_rows<true, true>(st, gulp, which, s) : launch_rows<true, false>(st, gulp, which, s);
+    k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
+    k_beam_sum<true><<<st.nbeam, kBeamT, 0, s>>>(st, which);
+    launches += 6;
+  };
+  // bandpass_flag: bandpass_correct (calc_bandpass_new, divide_by_bp), normalize_data
+  bandpass(true, 0, 1);
+  normalize(0);
   // calc_bandpass_new of the normalised data -> spectral flag
-  k_build_lut<<<lutg, 256, 0, s>>>(st, 2);
-  k_lane_partials<<<laneg, 256, 0, s>>>(gulp, st.lut, st.part, st.nchan, st.gulp);
-  k_lane_finish<<<fin_blocks, 256, 0, s>>>(st, 1);
+  k_build_lut<<<lutg, 256, 0, s>>>(st, 2, -1);
+  bandpass(false, 1, 3);
+  if (e != cudaSuccess) return e;
   if (st.nscrunch > 0) {
-    count_launches(11 + extra);
+    count_launches(launches + 1);
     return scrunch_planes(st, gulp, plain, R, wpos, dpos, s);
   }
-  // apply_scrunch(8,8,100,flag=0,ts=1): bandpass_correct ...
-  k_build_lut<<<lutg, 256, 0, s>>>(st, 3);
-  k_lane_partials<<<laneg, 256, 0, s>>>(gulp, st.lut, st.part, st.nchan, st.gulp);
-  extra += lane_finish(st, 2, fin_blocks, s) - 1;
-  k_build_lut<<<lutg, 256, 0, s>>>(st, 4);
-  // ... ts_correct ...
-  k_ts<<<dim3((st.gulp + kTsT - 1) / kTsT, st.nbeam), kTsT, 0, s>>>(gulp, st);
-  // ... normalize_data
-  k_row_partials<false, true><<<rowg, kRowT, kLutSlice, s>>>(gulp, st, 1);
-  k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-  k_beam_sum<false><<<st.nbeam, kBeamT, 0, s>>>(st, 1);
-  k_row_partials<true, true><<<rowg, kRowT, kLutSlice, s>>>(gulp, st, 1);
-  k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-  k_beam_sum<true><<<st.nbeam, kBeamT, 0, s>>>(st, 1);
+  // apply_scrunch(8,8,100,flag=0,ts=1): bandpass_correct, ts_correct, normalize_data
+  bandpass(false, 2, 4);
+  if (e == cudaSuccess) e = launch_ts(st, gulp, s);
+  normalize(1);
+  if (e != cudaSuccess) return e;
   // transpose_output into the ring
   k_flag_out<<<dim3(st.nchan / kOutC, (st.gulp + kOutT - 1) / kOutT, st.nbeam), 256, 0, s>>>(gulp, st, plain,
                                                                                          R, wpos, dpos);
-  count_launches(24 + extra);
+  count_launches(launches + 3);
   return cudaGetLastError();
 }
 }  // namespace

@@ -34,6 +34,9 @@ constexpr int kDedispThreads = kPackS;
 constexpr int kDedispGroup = 8;
 
 // ------------------------------------------------------------- flagger
+// Channels of a slice of the flagger's level tables.
+constexpr int kLutSl = 128;
+constexpr int lut_slices(int nchan) { return (nchan + kLutSl - 1) / kLutSl; }
 struct FlagState {
   int nbeam, nchan, gulp;
   float spec_min, spec_max;
@@ -42,10 +45,11 @@ struct FlagState {
   float *rowval;            // [nbeam][nchan] per-channel row statistic
   float *scal;              // [nbeam][8] mean1 std1 mean2 std2
   __half *hsc;              // [nbeam][8] half(-mean1) half(1/std1) ...
-  __half *lut;              // [nbeam][nchan][256]
+  __half *lut;              // [nbeam][lut_slices(nchan)][256][kLutSl]
   uint8_t *flag2;           // [nbeam][nchan] spectral flag decision
   float *ts;                // [nbeam][gulp]
   __half *hts;              // [nbeam][gulp]
+  float2 *tdiv;             // [nbeam][gulp] hts and its reciprocal, as floats
   // SCRUNCH entries (apply_scrunch with flag = 1, flagger.cu:271-343): the
   // data stop being a function of (channel, u8 level), so the flagger then
   // keeps fp16 planes [nbeam][nchan][gulp] (channel-major) instead

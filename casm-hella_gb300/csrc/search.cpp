@@ -423,10 +423,11 @@ hella_status hella_create(hella_ctx **out, const hella_params *p) {
   DA(f.rowval, nb * nch * 4);
   DA(f.scal, nb * 8 * 4);
   DA(f.hsc, nb * 8 * 2);
-  DA(f.lut, nb * nch * 256 * 2);
+  DA(f.lut, nb * hg::lut_slices(nch) * hg::kLutSl * 256 * 2);
   DA(f.flag2, nb * nch);
   DA(f.ts, nb * p->gulp * 4);
   DA(f.hts, nb * p->gulp * 2);
+  DA(f.tdiv, nb * p->gulp * 8);
   hg::flag_scrunch_params(*p, &f);
   if (p->nscrunch > 0 || f.f16_input) {
     DA(f.P, nb * nch * p->gulp * 2);
