@@ -898,6 +898,10 @@ hella_status hella_batch_create(hella_batch **out, const hella_batch_params *bp)
   DA(f.ts, (size_t)nb * p->gulp * 4);
   DA(f.hts, (size_t)nb * p->gulp * 2);
   DA(f.tdiv, (size_t)nb * p->gulp * 8);
+  if (hg::flag_prepare(f) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(HELLA_ERR_CUDA);
+  }
   hg::flag_scrunch_params(*p, &f);
   if (p->nscrunch > 0 || f.f16_input) {
     DA(f.P, (size_t)nb * nch * p->gulp * 2);

@@ -115,18 +115,6 @@ __global__ void __launch_bounds__(256) k_build_lut(FlagState st, int stage, int 
     row[v * kLutSl] = chain_value(stage, v, ch);
 }
 
-// Stages the table of channels c0 .. c0 + NC - 1 of beam b (within one slice) as
-// lut_s[level * NC + channel] with 16-byte loads of eight channels of a level;
-// channels past the slice's last hold anything.
-template <int NC>
-__device__ __forceinline__ void load_lut_slice(__half *lut_s, __half *lut, int nchan, int b, int c0) {
-  const __half *src = lut_row(lut, nchan, b, c0, 0);
-  for (int i = threadIdx.x; i < NC * 32; i += blockDim.x) {
-    const int v = i / (NC / 8), k = 8 * (i % (NC / 8));
-    *reinterpret_cast<uint4 *>(lut_s + v * NC + k) = *reinterpret_cast<const uint4 *>(src + v * kLutSl + k);
-  }
-}
-
 // a / b for half-precision a, b with r = 1 / b rounded: one correction step
 // after a first product (P. Markstein, IBM J. Res. Dev. 34, 1990) gives the
 // float quotient, whose rounding to half is the half quotient (24 bits are twice
@@ -539,6 +527,9 @@ __global__ void __launch_bounds__(32 * kTsWarps) k_ts(const uint8_t *__restrict_
   }
 }
 
+// The launchers below with a null gulp only allow their kernel the most dynamic
+// shared memory that any gulp takes, the same for all (flag_prepare).
+
 // Launches k_sums.  Lane sums have 32 chains a channel: with fewer than four
 // warps an SM in all, a lane takes two channels (twice the warps; levels are added
 // two to a word anyway), blocks are as small as spreads them over the SMs and
@@ -548,10 +539,9 @@ __global__ void __launch_bounds__(32 * kTsWarps) k_ts(const uint8_t *__restrict_
 template <int MOD, bool VAR, bool TS, bool RAW, int CH, int ROWS, int AHEAD>
 cudaError_t launch_sums(const FlagState &st, const uint8_t *gulp, int which, int nw, int per, cudaStream_t s) {
   const auto k = k_sums<MOD, VAR, TS, RAW, CH, ROWS, AHEAD>;
-  const int smem = (RAW ? 0 : kLutBytes) + nw * (AHEAD + 1) * sum_stage(ROWS, CH, TS);
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  k<<<dim3(lut_slices(st.nchan), MOD / (nw * CH / 4 * per), st.nbeam), 32 * nw, smem, s>>>(gulp, st, which, per);
+  auto smem = [](int warps) { return (RAW ? 0 : kLutBytes) + warps * (AHEAD + 1) * sum_stage(ROWS, CH, TS); };
+  if (!gulp) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(kSumWarps));
+  k<<<dim3(lut_slices(st.nchan), MOD / (nw * CH / 4 * per), st.nbeam), 32 * nw, smem(nw), s>>>(gulp, st, which, per);
   return cudaSuccess;
 }
 template <bool RAW>
@@ -573,9 +563,7 @@ cudaError_t launch_rows(const FlagState &st, const uint8_t *gulp, int which, cud
 // Launches k_ts with as many warps a block as fill whole rounds of one block
 // an SM (the table ring leaves no room for two), and four at least to copy.
 cudaError_t launch_ts(const FlagState &st, const uint8_t *gulp, cudaStream_t s) {
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_ts, cudaFuncAttributeMaxDynamicSharedMemorySize, ts_smem(kTsWarps));
-  if (e != cudaSuccess) return e;
+  if (!gulp) return cudaFuncSetAttribute(k_ts, cudaFuncAttributeMaxDynamicSharedMemorySize, ts_smem(kTsWarps));
   const long per = st.gulp / 32, warps = per * st.nbeam;
   const long rounds = (warps + 152 * kTsWarps - 1) / (152 * kTsWarps);
   const int nw = (int)((warps + 152 * rounds - 1) / (152 * rounds));
@@ -585,54 +573,141 @@ cudaError_t launch_ts(const FlagState &st, const uint8_t *gulp, cudaStream_t s) 
 }
 
 // transpose_output (transpose.cu:321-331): u8 = trunc(clamp(255/14 (x+4))).
+constexpr float kRequant = 255.f / 14.f;
 __device__ __forceinline__ uint8_t requant(__half h) {
-  float v = __half2float(h);
-  const float scf = 255.f / 14.f;
-  v = __fmul_rn(scf, __fadd_rn(v, 4.f));
+  float v = __fmul_rn(kRequant, __fadd_rn(__half2float(h), 4.f));
   if (v < 0.f) v = 0.f;
   if (v > 255.f) v = 255.f;
   return (uint8_t)v;
 }
+// The same bytes as the lowest of lo and hi: x is held in [-4, 10 + 1/128], whose
+// ends give 0 and 255 (NaN gives 0), and 2^23 plus the product, rounded toward zero
+// once, ends in its whole part (checked for every half: test_requant_every_half).
+__device__ __forceinline__ void requant2(__half2 x, uint32_t &lo, uint32_t &hi) {
+  x = __hmin2(__hmax2(x, __float2half2_rn(-4.f)), __float2half2_rn(10.0078125f));
+  lo = __float_as_uint(__fmaf_rz(kRequant, __fadd_rn(__low2float(x), 4.f), 8388608.f));
+  hi = __float_as_uint(__fmaf_rz(kRequant, __fadd_rn(__high2float(x), 4.f), 8388608.f));
+}
 
 // Final stage: divide_by_ts, normalize_data, requantise, and write the
-// channel-major ring.  Block = 32 channels x kOutT samples: the channels'
-// table slice is staged in shared memory (as in k_lane_partials), each
-// thread maps samples of one channel into a channel-major byte tile
-// (row stride kOutT + 4: conflict-free both ways), and the tile leaves as
-// 4-byte words, 128 bytes of one channel per warp.  The ring position of a
-// gulp (and R) are multiples of 32, so no word straddles the ring's end.
-constexpr int kOutT = 512, kOutC = 32;
-__global__ void __launch_bounds__(256) k_flag_out(const uint8_t *__restrict__ gulp, FlagState st,
-                                                  uint8_t *__restrict__ plain, long R, long wpos,
-                                                  const GulpPos *dpos) {
+// channel-major ring.  A block takes a slice of 128 channels, its table in
+// shared memory for all of its `run` tiles of kOutT samples.  Warps hold samples,
+// lanes four channels, looked up as in k_sums; a lane's four samples of four
+// channels become four words of four samples by byte permutes, go through a
+// shared tile ([channel within lane][lane], an odd number of words a row:
+// conflict-free both ways) and leave as 128 bytes of one channel a warp.  The
+// next tile's words are loaded before the current one's are mapped.  The ring
+// position of a gulp (and R) are multiples of 32, so no word straddles the
+// ring's end.  Bound by instruction issue (about 20 a sample): 8 beams x 32,768 samples
+// x 1024 channels 198 us, 424 us with one channel a lane and half-precision
+// division.
+constexpr int kOutT = 128, kOutRows = kOutT / 8;  // samples a tile, a warp
+constexpr int kOutPitch = kOutT / 4 + 1;          // words a tile row
+constexpr int kOutTile = 4 * 32 * kOutPitch * 4, kOutTd = 2 * kOutT * (int)sizeof(float2);
+constexpr int kOutSmem = kLutBytes + kOutTile + kOutTd;
+__global__ void __launch_bounds__(256, 2) k_flag_out(const uint8_t *__restrict__ gulp, FlagState st,
+                                                     uint8_t *__restrict__ plain, long R, long wpos,
+                                                     const GulpPos *dpos, int run) {
   if (dpos) wpos = dpos->wpos;
-  __shared__ __align__(16) __half lut_s[256][kOutC];
-  __shared__ __align__(16) uint8_t tile[kOutC][kOutT + 4];
-  const int b = blockIdx.z, c0 = blockIdx.x * kOutC, t0 = blockIdx.y * kOutT;
-  const int nchan = st.nchan, w = st.gulp, tid = threadIdx.x;
-  load_lut_slice<kOutC>(&lut_s[0][0], st.lut, nchan, b, c0);
-  __syncthreads();
-  const __half a2 = st.hsc[b * 8 + 2], m2 = st.hsc[b * 8 + 3];
-  const uint8_t *g = gulp + (size_t)b * w * nchan + c0;
-  const __half *hts = st.hts + (size_t)b * w;
-  const int cl = tid & 31, tr = tid >> 5;
-  const int nt = min(kOutT, w - t0);
+  extern __shared__ __align__(16) uint8_t out_s[];
+  uint32_t *tile = reinterpret_cast<uint32_t *>(out_s + kLutBytes);
+  const int b = blockIdx.z, c0 = blockIdx.x * kLutSl, nchan = st.nchan, w = st.gulp;
+  const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
+  const int tile0 = blockIdx.y * run, ntile = min(run, (w + kOutT - 1) / kOutT - tile0);
+  const uint8_t *lsrc = reinterpret_cast<const uint8_t *>(lut_row(st.lut, nchan, b, c0, 0));
 #pragma unroll 4
-  for (int tt = tr; tt < nt; tt += 8) {
-    const int t = t0 + tt;
-    __half x = __hdiv(lut_s[g[(size_t)t * nchan + cl]][cl], hts[t]);
-    x = __hmul(__hadd(x, a2), m2);
-    tile[cl][tt] = requant(x);
-  }
-  __syncthreads();
+  for (int i = tid * 16; i < kLutBytes; i += 256 * 16) copy_async<16>(out_s + i, lsrc + i);
+  // this warp's samples of a tile: kOutRows from wi * kOutRows on; their words and divisors
+  float2 *td = reinterpret_cast<float2 *>(out_s + kLutBytes + kOutTile) + wi * kOutRows;
+  const bool mine = c0 + 4 * lane < nchan;
+  const uint8_t *g = gulp + ((size_t)b * w + tile0 * kOutT + wi * kOutRows) * nchan + c0 + 4 * lane;
+  uint32_t x[kOutRows] = {};
+  auto load = [&](int k) {
+    const int t = (tile0 + k) * kOutT + wi * kOutRows;
+    if (k < ntile && t < w) {  // w % 32 == 0: all of the warp's samples or none
+      if (mine)
+#pragma unroll
+        for (int r = 0; r < kOutRows; ++r) x[r] = *reinterpret_cast<const uint32_t *>(g + (size_t)r * nchan);
+      if (lane < kOutRows) copy_async<8>(td + (k & 1) * kOutT + lane, st.tdiv + (size_t)b * w + t + lane);
+      g += (size_t)kOutT * nchan;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load(0);
+  const __half2 a2 = __half2half2(st.hsc[b * 8 + 2]), m2 = __half2half2(st.hsc[b * 8 + 3]);
+  const bool hi = lane >= 16;  // channels 2, 3 of its four first
+  const uint32_t first = 8u * lane + (hi ? 4u : 0u), second = 8u * lane + (hi ? 0u : 4u);
   uint8_t *pb = plain + ((size_t)b * nchan + c0) * R;
-  const int nq = nt / 4;  // w % 32 == 0
-  for (int i = tid; i < kOutC * nq; i += 256) {
-    const int c = i / nq, q = i - c * nq;
-    long pos = wpos + t0 + 4 * q;
+  for (int k = 0; k < ntile; ++k) {
+    uint32_t cur[kOutRows];
+#pragma unroll
+    for (int r = 0; r < kOutRows; ++r) cur[r] = __byte_perm(x[r], x[r], hi ? 0x1032 : 0x3210);
+    load(k + 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // the table; the divisors; the tile's readers are done
+    const float2 *tdk = td + (k & 1) * kOutT;
+#pragma unroll
+    for (int r0 = 0; r0 < kOutRows; r0 += 4) {
+      uint32_t o[4][4];  // [sample][channel as taken]
+      auto map = [&](bool fast) {
+        __half2 sum = __half2half2(hzero());
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float2 t = tdk[r0 + r];
+          __half h[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            h[q] = *reinterpret_cast<const __half *>(
+                out_s + __byte_perm(cur[r0 + r], q < 2 ? first : second, 0x7704 + 16 * q) + 2 * (q & 1));
+#pragma unroll
+          for (int q = 0; q < 4; q += 2) {
+            __half2 p;
+            if (fast) {
+              p = __floats2half2_rn(div_step(__half2float(h[q]), t.x, t.y), div_step(__half2float(h[q + 1]), t.x, t.y));
+              sum = __hadd2(sum, p);
+            } else {
+              const __half th = __float2half_rn(t.x);
+              p = __halves2half2(__hdiv(h[q], th), __hdiv(h[q + 1], th));
+            }
+            requant2(__hmul2(__hadd2(p, a2), m2), o[r][q], o[r][q + 1]);
+          }
+        }
+        return __half2float(__low2half(sum)) + __half2float(__high2half(sum));
+      };
+      // a quotient that div_step does not give leaves the sum infinite or NaN
+      if (!(fabsf(map(true)) <= 1e30f)) map(false);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t lo = __byte_perm(o[0][q], o[1][q], 0x0040), hi2 = __byte_perm(o[2][q], o[3][q], 0x0040);
+        tile[((hi ? q ^ 2 : q) * 32 + lane) * kOutPitch + (wi * kOutRows + r0) / 4] = __byte_perm(lo, hi2, 0x5410);
+      }
+    }
+    __syncthreads();
+    const int t = (tile0 + k) * kOutT, nq = min(kOutT, w - t) / 4;  // w % 32 == 0
+    long pos = wpos + t + 4 * lane;
     if (pos >= R) pos -= R;
-    *reinterpret_cast<uint32_t *>(pb + (size_t)c * R + pos) = *reinterpret_cast<const uint32_t *>(&tile[c][4 * q]);
+    if (lane < nq) {
+      uint8_t *d = pb + (size_t)wi * R + pos;
+      const uint32_t *row = tile + ((wi & 3) * 32 + (wi >> 2)) * kOutPitch + lane;  // channel wi; wi + 8 is two lanes on
+      const int nc = min(kLutSl, nchan - c0);
+#pragma unroll 4
+      for (int c = wi; c < nc; c += 8, d += 8 * R, row += 2 * kOutPitch) *reinterpret_cast<uint32_t *>(d) = *row;
+    }
   }
+}
+static_assert(kOutT / 4 == 32, "a lane a word of a tile's row");
+
+// Launches k_flag_out with runs that leave four blocks an SM (two fit) where the
+// gulp has as many tiles.
+cudaError_t launch_out(const FlagState &st, const uint8_t *gulp, uint8_t *plain, long R, long wpos,
+                       const GulpPos *dpos, cudaStream_t s) {
+  if (!gulp) return cudaFuncSetAttribute(k_flag_out, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutSmem);
+  const int tiles = (st.gulp + kOutT - 1) / kOutT;
+  const long all = (long)tiles * lut_slices(st.nchan) * st.nbeam;
+  const int run = (int)std::max(1L, std::max(all / (4 * 152), (tiles + 65534L) / 65535));
+  k_flag_out<<<dim3(lut_slices(st.nchan), (tiles + run - 1) / run, st.nbeam), 256, kOutSmem, s>>>(gulp, st, plain, R,
+                                                                                              wpos, dpos, run);
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -954,12 +1029,23 @@ cudaError_t flag_impl(const FlagState &st, const void *gulp_in, uint8_t *plain, 
   normalize(1);
   if (e != cudaSuccess) return e;
   // transpose_output into the ring
-  k_flag_out<<<dim3(st.nchan / kOutC, (st.gulp + kOutT - 1) / kOutT, st.nbeam), 256, 0, s>>>(gulp, st, plain,
-                                                                                         R, wpos, dpos);
+  if ((e = launch_out(st, gulp, plain, R, wpos, dpos, s)) != cudaSuccess) return e;
   count_launches(launches + 3);
   return cudaGetLastError();
 }
 }  // namespace
+
+cudaError_t flag_prepare(const FlagState &st) {
+  cudaError_t e = launch_lanes<true>(st, nullptr, nullptr);
+  if (e == cudaSuccess) e = launch_lanes<false>(st, nullptr, nullptr);
+  if (e == cudaSuccess) e = launch_rows<false, false>(st, nullptr, 0, nullptr);
+  if (e == cudaSuccess) e = launch_rows<true, false>(st, nullptr, 0, nullptr);
+  if (e == cudaSuccess) e = launch_rows<false, true>(st, nullptr, 1, nullptr);
+  if (e == cudaSuccess) e = launch_rows<true, true>(st, nullptr, 1, nullptr);
+  if (e == cudaSuccess) e = launch_ts(st, nullptr, nullptr);
+  if (e == cudaSuccess) e = launch_out(st, nullptr, nullptr, 0, 0, nullptr, nullptr);
+  return e;
+}
 
 // The ring writers store 4-byte words: the ring length and every write
 // position (gulp starts) are multiples of 32 samples.

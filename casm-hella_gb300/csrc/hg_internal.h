@@ -70,6 +70,9 @@ constexpr int kMaxBpMedian = 63;
 // Largest SCRUNCH widths the box filter stages in shared memory.
 constexpr int kMaxScrunch = 64;
 
+// Once per state (nbeam, nchan and gulp set) before its first gulp: lets the kernels
+// that it takes use their shared memory on the current device.
+cudaError_t flag_prepare(const FlagState &st);
 // Runs the whole parity flagger for all beams of `gulp` (u8 [nbeam][gulp]
 // [nchan]) and writes the requantised output into the plain ring at ring
 // position `wpos` (mod R) of every beam.

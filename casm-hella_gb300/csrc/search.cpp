@@ -428,6 +428,10 @@ hella_status hella_create(hella_ctx **out, const hella_params *p) {
   DA(f.ts, nb * p->gulp * 4);
   DA(f.hts, nb * p->gulp * 2);
   DA(f.tdiv, nb * p->gulp * 8);
+  if (hg::flag_prepare(f) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(HELLA_ERR_CUDA);
+  }
   hg::flag_scrunch_params(*p, &f);
   if (p->nscrunch > 0 || f.f16_input) {
     DA(f.P, nb * nch * p->gulp * 2);

@@ -3,7 +3,7 @@ warps and rounds of blocks, short chains), bit for bit against the oracle."""
 import numpy as np
 import pytest
 
-from helpers import small_params
+from helpers import oracle_pipeline, small_params
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +34,36 @@ def test_flagger_edges(hella, oracle, nchan, gulp):
     assert same(st["ts"], ts)
     if not np.isnan(st["mean2"]):  # the byte of a NaN is not defined either
         assert np.array_equal(s.copy_window(0)[-gulp:], out)
+
+
+@pytest.mark.parametrize("gulp", [256, 288, 1056, 2080, 8480])
+def test_gulp_loop_odd_gulps(hella, oracle, gulp):
+    """Words packed over gulps that are no whole blocks and runs, round the ring: the
+    dedispersed planes of each gulp against the oracle's on the same window."""
+    p = small_params(nchan=96, gulp=gulp, df_mhz=-(468.75 - 375.0) / 96, dm_max=60.0)
+    s = hella.Search(hella.default_params(**p))
+    pl = oracle_pipeline(oracle, p)
+    rng = np.random.default_rng(gulp)
+    for g in range(pl.min_gulp + 3):
+        x = rng.integers(100, 156, (1, gulp, 96), dtype=np.uint8)
+        _, searched = s.process_gulp(x)
+        _, expected = pl.gulp_step(x)
+        assert searched == expected
+        if searched:
+            s.clear_peaks()
+            s.load_gulp(x)
+            s.fast_flagger()
+            s.dedisperse(0)
+            assert np.array_equal(s.copy_dedisp(), pl.search_window(s.copy_window(0), 0)["dd"]), g
+            break
+
+
+def test_requant_every_half():
+    """The output stage's clamp in half precision and its one rounding toward zero
+    against the reference's clamp and truncation, for every half."""
+    h = np.arange(65536, dtype=np.uint16).view(np.float16)
+    h = h[~np.isnan(h)].astype(np.float32)
+    scale = np.float32(255) / np.float32(14)
+    ref = np.clip(scale * (h + np.float32(4)), 0, 255).astype(np.uint8)
+    held = np.clip(h, np.float32(-4), np.float32(10.0078125)) + np.float32(4)
+    assert np.array_equal(np.floor(np.float64(scale) * held).astype(np.int64) & 255, ref)
