@@ -151,6 +151,7 @@ struct hella_batch {
   hg::FlagState fs{};
   float *d_dd = nullptr, *d_boxes = nullptr, *d_taps = nullptr, *d_ew = nullptr;
   int *d_tapoff = nullptr, *d_tapn = nullptr;
+  unsigned *d_done = nullptr;
   float *d_rowmean = nullptr, *d_rowmax = nullptr, *d_rowvar = nullptr, *d_stats = nullptr,
         *d_gate = nullptr;
   int *d_counts = nullptr, *d_offsets = nullptr, *d_total = nullptr, *d_active = nullptr,
@@ -315,6 +316,7 @@ hella_status upload_layout(hella_batch *b) {
     B.offsets = b->d_offsets + b->row_off[i];
     B.stats = b->d_stats + (size_t)i * b->z.nbox * 4;
     B.gate = b->d_gate + (size_t)i * 4;
+    B.done = b->d_done + (size_t)i * b->z.nbox;
     B.cand_i = b->d_cand_i + (size_t)i * cap;
     B.cand_v = b->d_cand_v + (size_t)i * cap;
     B.total = b->d_total + i;
@@ -898,6 +900,7 @@ hella_status hella_batch_create(hella_batch **out, const hella_batch_params *bp)
   DA(f.ts, (size_t)nb * p->gulp * 4);
   DA(f.hts, (size_t)nb * p->gulp * 2);
   DA(f.tdiv, (size_t)nb * p->gulp * 8);
+  DA(f.done, (size_t)nb * 4);
   if (hg::flag_prepare(f) != cudaSuccess) {
     cudaGetLastError();
     return fail(HELLA_ERR_CUDA);
@@ -921,6 +924,7 @@ hella_status hella_batch_create(hella_batch **out, const hella_batch_params *bp)
   DA(b->d_offsets, rw * 4);
   DA(b->d_stats, (size_t)nb * z.nbox * 16);
   DA(b->d_gate, (size_t)nb * 16);
+  DA(b->d_done, (size_t)nb * z.nbox * 4);
   DA(b->d_total, (size_t)nb * 4);
   DA(b->d_active, (size_t)nb * 4);
   DA(b->d_row_beam, rows * 4);
@@ -959,6 +963,8 @@ hella_status hella_batch_create(hella_batch **out, const hella_batch_params *bp)
       cudaMemset(b->d_ew, 0, (size_t)nb * nch * 4) != cudaSuccess ||
       cudaMemset(f.flagspec, 0, (size_t)nch * 4) != cudaSuccess ||
       cudaMemset(b->d_err, 0, 16) != cudaSuccess || cudaMemset(b->d_total, 0, (size_t)nb * 4) != cudaSuccess ||
+      cudaMemset(b->d_done, 0, (size_t)nb * z.nbox * 4) != cudaSuccess ||
+      cudaMemset(f.done, 0, (size_t)nb * 4) != cudaSuccess ||
       cudaDeviceSynchronize() != cudaSuccess) {
     cudaGetLastError();
     return fail(HELLA_ERR_CUDA);

@@ -22,6 +22,7 @@
 // so the output bytes equal the reference's on the same gulp.
 #include "hg_internal.h"
 #include "hella_search.h"
+#include "hg_ptx.h"
 
 #include <algorithm>
 #include <cmath>
@@ -82,8 +83,8 @@ __device__ __forceinline__ void put_bandpass(const FlagState &st, int mode, int 
 // 3 us, for 128 bytes a channel): every block does so for its own 32 channels, the
 // first of a column of blocks for all readers to come, and the values of its own
 // blocks come from shared memory.
-constexpr int kLutRows = 32, kLutC = 32;  // levels and channels a block
-__global__ void __launch_bounds__(256) k_build_lut(FlagState st, int stage, int fin) {
+constexpr int kLutC = 32;  // channels a block
+__global__ void __launch_bounds__(256) k_build_lut(FlagState st, int stage, int fin, int rows) {
   __shared__ float bp_s[kLutC];
   const int cl = threadIdx.x % kLutC, c0 = blockIdx.x * kLutC, b = blockIdx.z, wi = threadIdx.x / 32;
   const int bc0 = b * st.nchan + c0;
@@ -110,9 +111,14 @@ __global__ void __launch_bounds__(256) k_build_lut(FlagState st, int stage, int 
     ch.mul = st.hsc[b * 8 + 1];
   }
   __half *row = lut_row(st.lut, st.nchan, b, c0 + cl, 0);
-#pragma unroll
-  for (int v = blockIdx.y * kLutRows + wi, i = 0; i < kLutRows / 8; ++i, v += 8)
-    row[v * kLutSl] = chain_value(stage, v, ch);
+#pragma unroll 4
+  for (int v = wi; v < rows; v += 8) row[(blockIdx.y * rows + v) * kLutSl] = chain_value(stage, blockIdx.y * rows + v, ch);
+}
+// 8 levels a block, 32 where that still leaves two blocks an SM (1024 channels x 8 beams:
+// 9.2 us, 17.9 us with 8).
+void launch_lut(const FlagState &st, int stage, int fin, cudaStream_t s) {
+  const int rows = st.nchan / kLutC * st.nbeam * 8 >= 2 * 152 ? 32 : 8;
+  k_build_lut<<<dim3(st.nchan / kLutC, 256 / rows, st.nbeam), 256, 0, s>>>(st, stage, fin, rows);
 }
 
 // a / b for half-precision a, b with r = 1 / b rounded: one correction step
@@ -342,43 +348,36 @@ __global__ void k_lane_finish(FlagState st, int mode) {
 }
 
 // Thread 0 of the reference's 256-thread block: each warp's shuffle tree,
-// then warp totals 1..7 added in order, / nw.  One warp per channel.
-__global__ void k_row_finish(FlagState st) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= st.nbeam * st.nchan) return;
-  const float *p = st.part + (size_t)gw * 256;
-  float tot = 0.f;
-  for (int wi = 0; wi < 8; ++wi) {
-    float v = p[wi * 32 + lane];
-    for (int off = 16; off > 0; off /= 2) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
-    tot = wi == 0 ? v : __fadd_rn(tot, v);
-  }
-  if (lane == 0) st.rowval[gw] = __fdiv_rn(tot, (float)(256 * (st.gulp / 256)));
-}
-
-// calculate_stddev's host loops (normalization.cu:138-153): sequential sum
-// over channels, / nchan; the variance pass also forms the half-precision
-// normalisation constants of normalize_data (flagger.cu:205-206).  Block =
-// beam: the row values are staged in shared memory with coalesced loads,
-// thread 0 adds them in channel order.
+// then warp totals 1..7 added in order, / nw.  One warp per channel, a block's
+// channels of one beam (nchan % 32 == 0).  The last block of a beam then runs
+// calculate_stddev's host loop (normalization.cu:138-153): sequential sum over
+// channels, / nchan; the variance pass also forms the half-precision
+// normalisation constants of normalize_data (flagger.cu:205-206).  (A launch of
+// its own for that cost 3 to 9 us.)
 constexpr int kBeamT = 256, kMaxChan = 8192;  // the largest nchan accepted
 template <bool VAR>
-__global__ void __launch_bounds__(kBeamT) k_beam_sum(FlagState st, int which) {
-  __shared__ float rv_s[kMaxChan];
-  const int b = blockIdx.x;
-  const float *rv = st.rowval + (size_t)b * st.nchan;
-  for (int c = threadIdx.x; c < st.nchan; c += kBeamT) rv_s[c] = rv[c];
-  __syncthreads();
+__global__ void __launch_bounds__(kBeamT) k_row_finish(FlagState st, int which) {
+  const int c = blockIdx.x * (kBeamT / 32) + (threadIdx.x >> 5), b = blockIdx.y, lane = threadIdx.x & 31;
+  const float *p = st.part + ((size_t)b * st.nchan + c) * 256;
+  float v[8];
+#pragma unroll
+  for (int wi = 0; wi < 8; ++wi) v[wi] = p[wi * 32 + lane];
+#pragma unroll
+  for (int wi = 0; wi < 8; ++wi)
+    for (int off = 16; off > 0; off /= 2) v[wi] = __fadd_rn(v[wi], __shfl_down_sync(0xffffffffu, v[wi], off));
+  float tot = v[0];
+#pragma unroll
+  for (int wi = 1; wi < 8; ++wi) tot = __fadd_rn(tot, v[wi]);
+  float *rv = st.rowval + (size_t)b * st.nchan;
+  if (lane == 0) rv[c] = __fdiv_rn(tot, (float)(256 * (st.gulp / 256)));
+  if (!last_block(st.done + b, gridDim.x)) return;
+  float s = block_seq_sum(rv, st.nchan);
   if (threadIdx.x != 0) return;
-  float s = 0.f;
-  for (int c = 0; c < st.nchan; ++c) s = __fadd_rn(s, rv_s[c]);
   s = __fdiv_rn(s, (float)st.nchan);
   if (!VAR) {
     st.scal[b * 8 + 2 * which] = s;
   } else {
-    float sd = __fsqrt_rn(s);
-    float mean = st.scal[b * 8 + 2 * which];
+    const float sd = __fsqrt_rn(s), mean = st.scal[b * 8 + 2 * which];
     st.scal[b * 8 + 2 * which + 1] = sd;
     st.hsc[b * 8 + 2 * which] = __float2half_rn(-mean);
     st.hsc[b * 8 + 2 * which + 1] = __float2half_rn(__fdiv_rn(1.f, sd));
@@ -914,19 +913,18 @@ namespace {
 cudaError_t scrunch_planes(const FlagState &st, const void *gulp, uint8_t *plain, long R, long wpos,
                            const GulpPos *dpos, cudaStream_t s) {
   const int fin_blocks = (st.nbeam * st.nchan * 32 + 255) / 256;
+  const dim3 fing(st.nchan / (kBeamT / 32), st.nbeam);
   const size_t n = (size_t)st.nbeam * st.nchan * st.gulp;
   const int eb = (int)std::min<size_t>((n + 255) / 256, 152 * 16);
   const dim3 chg(st.nchan, st.nbeam);
   unsigned launches = 0;
   auto normalize = [&](int which) {
     k_plane_rows<false><<<chg, 256, 0, s>>>(st, which);
-    k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-    k_beam_sum<false><<<st.nbeam, kBeamT, 0, s>>>(st, which);
+    k_row_finish<false><<<fing, kBeamT, 0, s>>>(st, which);
     k_plane_rows<true><<<chg, 256, 0, s>>>(st, which);
-    k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-    k_beam_sum<true><<<st.nbeam, kBeamT, 0, s>>>(st, which);
+    k_row_finish<true><<<fing, kBeamT, 0, s>>>(st, which);
     k_plane_norm<<<eb, 256, 0, s>>>(st, which);
-    launches += 7;
+    launches += 5;
   };
   auto bandpass_correct = [&](int mode, const float *bp) {
     k_plane_lanes<<<fin_blocks, 256, 0, s>>>(st);
@@ -984,8 +982,8 @@ cudaError_t flag_impl(const FlagState &st, const void *gulp_in, uint8_t *plain, 
                       const GulpPos *dpos, cudaStream_t s) {
   if (st.f16_input) return scrunch_planes(st, gulp_in, plain, R, wpos, dpos, s);
   const uint8_t *gulp = static_cast<const uint8_t *>(gulp_in);
-  const dim3 lutg(st.nchan / kLutC, 256 / kLutRows, st.nbeam);
   const int fin_blocks = (st.nbeam * st.nchan * 32 + 255) / 256;
+  const dim3 fing(st.nchan / (kBeamT / 32), st.nbeam);
 
   cudaError_t e = cudaSuccess;
   unsigned launches = 0;
@@ -997,7 +995,7 @@ cudaError_t flag_impl(const FlagState &st, const void *gulp_in, uint8_t *plain, 
     const bool median = mode != 1 && st.bp_median > 1;
     if (median) launches += lane_finish(st, mode, fin_blocks, s);
     if (stage >= 0) {
-      k_build_lut<<<lutg, 256, 0, s>>>(st, stage, median ? -1 : mode);
+      launch_lut(st, stage, median ? -1 : mode, s);
       ++launches;
     } else if (!median) {
       launches += lane_finish(st, mode, fin_blocks, s);
@@ -1005,18 +1003,16 @@ cudaError_t flag_impl(const FlagState &st, const void *gulp_in, uint8_t *plain, 
   };
   auto normalize = [&](int which) {  // calculate_stddev: mean pass, variance pass
     if (e == cudaSuccess) e = which ? launch_rows<false, true>(st, gulp, which, s) : launch_rows<false, false>(st, gulp, which, s);
-    k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-    k_beam_sum<false><<<st.nbeam, kBeamT, 0, s>>>(st, which);
+    k_row_finish<false><<<fing, kBeamT, 0, s>>>(st, which);
     if (e == cudaSuccess) e = which ? launch_rows<true, true>(st, gulp, which, s) : launch_rows<true, false>(st, gulp, which, s);
-    k_row_finish<<<fin_blocks, 256, 0, s>>>(st);
-    k_beam_sum<true><<<st.nbeam, kBeamT, 0, s>>>(st, which);
-    launches += 6;
+    k_row_finish<true><<<fing, kBeamT, 0, s>>>(st, which);
+    launches += 4;
   };
   // bandpass_flag: bandpass_correct (calc_bandpass_new, divide_by_bp), normalize_data
   bandpass(true, 0, 1);
   normalize(0);
   // calc_bandpass_new of the normalised data -> spectral flag
-  k_build_lut<<<lutg, 256, 0, s>>>(st, 2, -1);
+  launch_lut(st, 2, -1, s);
   bandpass(false, 1, 3);
   if (e != cudaSuccess) return e;
   if (st.nscrunch > 0) {

@@ -50,6 +50,7 @@ struct FlagState {
   float *ts;                // [nbeam][gulp]
   __half *hts;              // [nbeam][gulp]
   float2 *tdiv;             // [nbeam][gulp] hts and its reciprocal, as floats
+  unsigned *done;           // [nbeam] blocks finished of a pass (0 between passes)
   // SCRUNCH entries (apply_scrunch with flag = 1, flagger.cu:271-343): the
   // data stop being a function of (channel, u8 level), so the flagger then
   // keeps fp16 planes [nbeam][nchan][gulp] (channel-major) instead
@@ -298,6 +299,7 @@ struct SmoothBeam {
   int4 *cand_i;             // [cap] beam, dm_idx, width, samp
   float *cand_v;            // [cap] normalised value
   int *total;               // [1] candidates written so far (capped at cap)
+  unsigned *done;           // [nbox] rows finished of a pass (0 between passes)
   const int *active;        // searched this gulp (0: every kernel skips the beam)
   int h;                    // rows: ndms - 2
   int row0;                 // first global row of the beam

@@ -131,4 +131,56 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
       : "memory");
 }
 
+// Whether this block is the last of n to get here, once per launch: true in every
+// thread of that block, which then sees what the others wrote before (read it past
+// the L1).  *done is 0 before and after.  Called by a whole block.
+__device__ __forceinline__ bool last_block(unsigned *done, unsigned n) {
+  __shared__ bool last_s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();  // after the barrier: all the block's writes
+    last_s = atomicAdd(done, 1u) == n - 1;
+    if (last_s) *done = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return last_s;
+}
+
+// Sequential sum of v[0 .. n) in index order in thread 0 (others: anything); the
+// block stages kSeqChunk values at a time in shared memory, and sixteen are read
+// ahead of the chain of additions, which is what bounds it.
+constexpr int kSeqChunk = 2048;
+__device__ __forceinline__ float block_seq_sum(const float *v, int n) {
+  __shared__ __align__(16) float chunk_s[kSeqChunk + 16];
+  float s = 0.f;
+  for (int c0 = 0; c0 < n; c0 += kSeqChunk) {
+    const int m = min(kSeqChunk, n - c0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += blockDim.x) chunk_s[i] = __ldcg(v + c0 + i);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const float4 *q = reinterpret_cast<const float4 *>(chunk_s);  // read ahead past m, within the chunk
+      float4 cur[4], next[4];
+      auto add = [&](const float4(&w)[4]) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, w[k].x), w[k].y), w[k].z), w[k].w);
+      };
+#pragma unroll
+      for (int k = 0; k < 4; ++k) cur[k] = q[k];
+      int i = 0;
+      for (; i + 32 <= m; i += 32) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) next[k] = q[i / 4 + 4 + k];
+        add(cur);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) cur[k] = q[i / 4 + 8 + k];
+        add(next);
+      }
+      for (; i < m; ++i) s = __fadd_rn(s, chunk_s[i]);
+    }
+  }
+  return s;
+}
+
 }  // namespace hg

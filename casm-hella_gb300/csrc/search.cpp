@@ -113,6 +113,7 @@ struct hella_ctx {
   size_t dev_bytes = 0;
   std::vector<void *> dallocs, hallocs;
   uint8_t *d_gulp = nullptr, *d_plain = nullptr;
+  unsigned *d_done = nullptr;
   uint32_t *d_packed = nullptr;
   hg::FlagState fs{};
   float *d_dd = nullptr, *d_boxes = nullptr, *d_taps = nullptr;
@@ -206,6 +207,7 @@ hella_status upload_beam(hella_ctx *c, int cap, int beam_id) {
   B.rowvar = c->d_rowvar;
   B.stats = c->d_stats;
   B.gate = c->d_gate;
+  B.done = c->d_done;
   B.counts = c->d_counts;
   B.offsets = c->d_offsets;
   B.cand_i = c->d_cand_i;
@@ -428,6 +430,7 @@ hella_status hella_create(hella_ctx **out, const hella_params *p) {
   DA(f.ts, nb * p->gulp * 4);
   DA(f.hts, nb * p->gulp * 2);
   DA(f.tdiv, nb * p->gulp * 8);
+  DA(f.done, nb * 4);
   if (hg::flag_prepare(f) != cudaSuccess) {
     cudaGetLastError();
     return fail(HELLA_ERR_CUDA);
@@ -447,6 +450,7 @@ hella_status hella_create(hella_ctx **out, const hella_params *p) {
   DA(c->d_rowvar, c->nbox * h * 4);
   DA(c->d_stats, c->nbox * 16);
   DA(c->d_gate, 16);
+  DA(c->d_done, c->nbox * 4);
   DA(c->d_flagspec, nch * 4);
   f.flagspec = c->d_flagspec;
   DA(c->d_counts, c->nbox * h * 4);
@@ -478,7 +482,8 @@ hella_status hella_create(hella_ctx **out, const hella_params *p) {
       cudaMemset(c->d_plain, 0, nb * nch * R) != cudaSuccess ||
       cudaMemset(c->d_packed, 0, nb * nch * R * 4) != cudaSuccess ||
       cudaMemset(c->d_flagspec, 0, nch * 4) != cudaSuccess ||
-      cudaMemset(c->d_err, 0, 16) != cudaSuccess ||
+      cudaMemset(c->d_err, 0, 16) != cudaSuccess || cudaMemset(c->d_done, 0, c->nbox * 4) != cudaSuccess ||
+      cudaMemset(f.done, 0, nb * 4) != cudaSuccess ||
       cudaMemset(c->d_row_beam, 0, (size_t)c->ndms * 4) != cudaSuccess ||
       cudaMemcpy(c->d_active, &kOne, 4, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaDeviceSynchronize() != cudaSuccess) {

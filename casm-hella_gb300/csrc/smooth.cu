@@ -24,6 +24,7 @@
 // variance.  Row maxima let the peak pass skip rows that cannot hold
 // a candidate.
 #include "hg_internal.h"
+#include "hg_ptx.h"
 
 #include <algorithm>
 
@@ -433,40 +434,58 @@ __global__ void __launch_bounds__(kLT, 6) k_firL(SmoothArgs a, int bend) {
   if (tid < 32) row_finish(B, b, r, out_s, out_s[256 + (tid & 3)], 256 * (nout / 256));
 }
 
-// Sequential sum of v[0..n) in index order (the reference's host loop),
-// in thread 0 of a kFin-thread block: the block stages kFinChunk values at
-// a time in shared memory with coalesced loads, thread 0 adds them.
-constexpr int kFin = 256, kFinChunk = 4096;
-__device__ float block_seq_sum(const float *v, int n, float *chunk_s) {
-  float s = 0.f;
-  for (int c0 = 0; c0 < n; c0 += kFinChunk) {
-    const int m = min(kFinChunk, n - c0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < m; i += kFin) chunk_s[i] = v[c0 + i];
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int i = 0; i < m; ++i) s = __fadd_rn(s, chunk_s[i]);
-  }
-  return s;
-}
+constexpr int kFin = 256;
 
 // Host loop of calculate_stddev (normalization.cu:138-142): sequential over
 // rows, / height.  Block = (beam, width of the launch).
 __global__ void __launch_bounds__(kFin) k_mean_finish(SmoothArgs a) {
-  __shared__ float chunk_s[kFinChunk];
   const SmoothBeam &B = a.beams[blockIdx.x];
   const int j = blockIdx.y;
   if (!*B.active) return;
   const int b = a.w0 + j, h = B.h;
-  const float s = block_seq_sum(B.rowmean + (size_t)b * h, h, chunk_s);
+  const float s = block_seq_sum(B.rowmean + (size_t)b * h, h);
   if (threadIdx.x == 0) B.stats[b * 4 + 0] = __fdiv_rn(s, (float)h);
+}
+
+// The host loop over rows for one (beam, width b): variance -> std and the
+// normalisation constants.  NORM0: the gate statistics of the normalised
+// width-0 plane.  By a whole block.
+template <bool NORM0, bool VAR>
+__device__ __forceinline__ void stat_finish(const SmoothArgs &a, const SmoothBeam &B, int b) {
+  float m = block_seq_sum(B.rowvar + (size_t)b * B.h, B.h);
+  if (threadIdx.x != 0) return;
+  m = __fdiv_rn(m, (float)B.h);
+  if (NORM0) {
+    if (!VAR) {
+      B.gate[0] = m;
+    } else {
+      const float sig = __fsqrt_rn(m);
+      B.gate[1] = sig;
+      B.gate[2] = __fmul_rn(a.snr, sig);
+      B.gate[3] = (a.nogate || (sig < 5 && (double)sig > 0.1)) ? 1.f : 0.f;  // definitions.h:66,71-72
+    }
+  } else {
+    const float sd = __fsqrt_rn(m), mu = B.stats[b * 4 + 0];
+    B.stats[b * 4 + 1] = sd;
+    B.stats[b * 4 + 2] = -1.0f * mu;
+    B.stats[b * 4 + 3] = __fdiv_rn(1.0f, sd);
+  }
+}
+
+// stat_finish by itself.  Block = (beam, width of the launch).
+template <bool NORM0, bool VAR>
+__global__ void __launch_bounds__(kFin) k_stat_finish(SmoothArgs a) {
+  const SmoothBeam &B = a.beams[blockIdx.x];
+  if (*B.active) stat_finish<NORM0, VAR>(a, B, NORM0 ? 0 : a.w0 + (int)blockIdx.y);
 }
 
 // computeRowVariances over one row of one width plane.  NORM0: the
 // normalised width-0 plane (find_peaks' sigma, peaks.cu:171-178), which
-// needs width 0 in the launch (w0 == 0).
-template <bool NORM0, bool VAR>
-__global__ void __launch_bounds__(kT) k_row_stat(SmoothArgs a) {
+// needs width 0 in the launch (w0 == 0).  FIN: the last row's block of a (beam,
+// width) runs stat_finish.  Bound by the memory: 2286 rows x 65,536 x 9 widths 813 us
+// (6.9 TB/s).
+template <bool NORM0, bool VAR, bool FIN>
+__global__ void __launch_bounds__(kT, !NORM0 && !FIN ? 8 : 6) k_row_stat(SmoothArgs a) {
   __shared__ float p_s[kT];
   int r;
   const SmoothBeam &B = row_beam(a, blockIdx.x, &r);
@@ -476,9 +495,10 @@ __global__ void __launch_bounds__(kT) k_row_stat(SmoothArgs a) {
   const int nwcol = 256 * (a.ntime_out / 256);
   const float *st = B.stats + b * 4;
   const float mean = NORM0 ? B.gate[0] : st[0];
+  const float norm[4] = {0.f, NORM0 ? st[1] : 0.f, NORM0 ? st[2] : 0.f, NORM0 ? st[3] : 0.f};  // normv's, read once
   float s = 0.f;
   auto add = [&](float v) {
-    if (NORM0) v = normv(v, st);
+    if (NORM0) v = normv(v, norm);
     if (VAR) {
       const float d = __fsub_rn(v, mean);
       s = __fmaf_rn(d, d, s);
@@ -503,35 +523,22 @@ __global__ void __launch_bounds__(kT) k_row_stat(SmoothArgs a) {
     const float tot = block256_tree(p_s);
     if (tid == 0) B.rowvar[(size_t)b * h + r] = __fdiv_rn(tot, (float)nwcol);
   }
+  if (FIN && last_block(B.done + b, (unsigned)h)) stat_finish<NORM0, VAR>(a, B, b);
 }
 
-// Per (beam, width): variance -> std and the normalisation constants.
-// NORM0: the gate statistics of the normalised width-0 plane.
+// A pass and the loop over its rows: one launch where the rows are few (512
+// channels x 16,384 samples, 3300 row blocks: 39 us for the two launches, 37 us for one), two
+// where waiting for the count of rows done holds blocks back more than a launch
+// costs (16 beams x 8192 samples: 508 + 10 us, 540 us).
 template <bool NORM0, bool VAR>
-__global__ void __launch_bounds__(kFin) k_stat_finish(SmoothArgs a) {
-  __shared__ float chunk_s[kFinChunk];
-  const SmoothBeam &B = a.beams[blockIdx.x];
-  const int j = NORM0 ? 0 : blockIdx.y;
-  if (!*B.active) return;
-  const int b = NORM0 ? 0 : a.w0 + j, h = B.h;
-  float s = block_seq_sum(B.rowvar + (size_t)b * h, h, chunk_s);
-  if (threadIdx.x != 0) return;
-  s = __fdiv_rn(s, (float)h);
-  if (NORM0) {
-    if (!VAR) {
-      B.gate[0] = s;
-    } else {
-      const float sig = __fsqrt_rn(s);
-      B.gate[1] = sig;
-      B.gate[2] = __fmul_rn(a.snr, sig);
-      B.gate[3] = (a.nogate || (sig < 5 && (double)sig > 0.1)) ? 1.f : 0.f;  // definitions.h:66,71-72
-    }
-  } else {
-    const float sd = __fsqrt_rn(s), mean = B.stats[b * 4 + 0];
-    B.stats[b * 4 + 1] = sd;
-    B.stats[b * 4 + 2] = -1.0f * mean;
-    B.stats[b * 4 + 3] = __fdiv_rn(1.0f, sd);
+unsigned row_stat(const SmoothArgs &a, int nw, cudaStream_t s) {
+  if ((long)a.nrows * nw <= 4096) {
+    k_row_stat<NORM0, VAR, true><<<dim3(a.nrows, nw), kT, 0, s>>>(a);
+    return 1;
   }
+  k_row_stat<NORM0, VAR, false><<<dim3(a.nrows, nw), kT, 0, s>>>(a);
+  k_stat_finish<NORM0, VAR><<<dim3(a.nbeam, nw), kFin, 0, s>>>(a);
+  return 2;
 }
 
 // Unnormalised planes (hella_smooth(ctx, 0)): stats zero for the widths.
@@ -548,7 +555,7 @@ __global__ void __launch_bounds__(kT) k_count(SmoothArgs a) {
   const SmoothBeam &B = row_beam(a, blockIdx.x, &r);
   const int j = blockIdx.y, b = a.w0 + j, h = B.h, tid = threadIdx.x;
   const size_t row = (size_t)b * h + r;
-  const float *st = B.stats + b * 4;
+  const float st[4] = {0.f, B.stats[b * 4 + 1], B.stats[b * 4 + 2], B.stats[b * 4 + 3]};  // normv's, read once
   const float thr = B.gate[2];
   // normalisation is monotonic, so the row maximum decides the whole row
   if (!*B.active || B.gate[3] == 0.f || !(normv(B.rowmax[row], st) > thr)) {
@@ -579,88 +586,93 @@ __global__ void __launch_bounds__(kT) k_count(SmoothArgs a) {
 
 // Per beam: exclusive scan of the row counts of the launch's widths in
 // (width, row) order, after the candidates of earlier widths; the beam's
-// total is capped at its cap.
+// total is capped at its cap.  1024 rows at a time, neighbouring ones in
+// neighbouring threads, warp sums by shuffles.
 __global__ void __launch_bounds__(1024) k_scan(SmoothArgs a) {
-  __shared__ int s_s[1024];
+  __shared__ int w_s[32];
   const SmoothBeam &B = a.beams[blockIdx.x];
   if (!*B.active) return;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nrows = a.nw * B.h;
-  int *counts = B.counts + (size_t)a.w0 * B.h, *offsets = B.offsets + (size_t)a.w0 * B.h;
-  const int base = B.total[0];
-  const int per = (nrows + 1023) / 1024;
-  const int lo = min(nrows, tid * per), hi = min(nrows, lo + per);
-  int sum = 0;
-  for (int i = lo; i < hi; ++i) sum += counts[i];
-  s_s[tid] = sum;
-  __syncthreads();
-  for (int off = 1; off < 1024; off *= 2) {
-    int v = tid >= off ? s_s[tid - off] : 0;
+  const int *counts = B.counts + (size_t)a.w0 * B.h;
+  int *offsets = B.offsets + (size_t)a.w0 * B.h;
+  int base = B.total[0];
+  int next = tid < nrows ? counts[tid] : 0;
+  for (int i0 = 0; i0 < nrows; i0 += 1024) {
+    const int i = i0 + tid, c = next;
+    next = i + 1024 < nrows ? counts[i + 1024] : 0;
+    int v = c;
+    for (int off = 1; off < 32; off *= 2) {
+      const int u = __shfl_up_sync(0xffffffffu, v, off);
+      if (lane >= off) v += u;
+    }
+    __syncthreads();  // the sums of the round before have been read
+    if (lane == 31) w_s[warp] = v;
     __syncthreads();
-    s_s[tid] += v;
-    __syncthreads();
+    int t = w_s[lane];
+    for (int off = 1; off < 32; off *= 2) {
+      const int u = __shfl_up_sync(0xffffffffu, t, off);
+      if (lane >= off) t += u;
+    }
+    const int before = __shfl_sync(0xffffffffu, t, (warp + 31) & 31);
+    if (i < nrows) offsets[i] = base + v - c + (warp ? before : 0);
+    base += __shfl_sync(0xffffffffu, t, 31);
   }
-  int run = base + s_s[tid] - sum;
-  for (int i = lo; i < hi; ++i) {
-    offsets[i] = run;
-    run += counts[i];
-  }
-  __syncthreads();
-  if (tid == 1023) B.total[0] = min(base + s_s[1023], B.cap);
+  if (tid == 0) B.total[0] = min(base, B.cap);
 }
 
-// Ordered compaction of one row's candidates, kWR chunks of 256 columns a
-// round: every thread reads one column of each chunk, the warps' hit
-// counts of the round are published once, and each hit is written at the
-// row's offset + the hits of earlier chunks + earlier warps of its chunk +
-// earlier lanes (column order).
-constexpr int kWR = 4;
-__global__ void __launch_bounds__(kT) k_write(SmoothArgs a) {
-  __shared__ int w_s[kWR][kT / 32];
+// Ordered compaction of one row's candidates, kWCols columns a round: a warp
+// takes a contiguous eighth of them, kWN values a thread loaded at once, the warps'
+// hits are published once a round, and a hit is written at the row's offset + the
+// hits of earlier rounds, warps, 32-column groups and lanes.  Bound by the loads'
+// latency on the few rows that have hits (16 or 32 values a thread leave too few
+// blocks an SM for the many rows that have none): 512 channels x 16,384 samples 15 us,
+// 47 us with 1024 columns and two barriers a round.
+constexpr int kWN = 8, kWCols = kWN * kT;
+__global__ void __launch_bounds__(kT, 8) k_write(SmoothArgs a) {
+  __shared__ int w_s[2][kT / 32];
   int r;
   const SmoothBeam &B = row_beam(a, blockIdx.x, &r);
   const int j = blockIdx.y, b = a.w0 + j, h = B.h, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const size_t row = (size_t)b * h + r;
   if (!*B.active || B.counts[row] == 0 || B.offsets[row] >= B.cap) return;
-  const float *st = B.stats + b * 4;
+  const float st[4] = {0.f, B.stats[b * 4 + 1], B.stats[b * 4 + 2], B.stats[b * 4 + 3]};  // normv's, read once
   const float thr = B.gate[2];
   const float *x = B.boxes + ((size_t)j * h + r) * a.ntime_out;
   int base = B.offsets[row];  // the same in every thread
-  for (int cs = 0; cs < a.ntime_out && base < B.cap; cs += kWR * kT) {
-    float v[kWR];
-    unsigned bal[kWR];
+  for (int c0 = 0, k = 0; c0 < a.ntime_out && base < B.cap; c0 += kWCols, k ^= 1) {
+    const int w0 = c0 + warp * (kWCols / (kT / 32));
+    float v[kWN];
 #pragma unroll
-    for (int m = 0; m < kWR; ++m) {
-      const int col = cs + m * kT + tid;
-      v[m] = col < a.ntime_out ? normv(x[col], st) : 0.f;
+    for (int m = 0; m < kWN; ++m) v[m] = w0 + m * 32 + lane < a.ntime_out ? x[w0 + m * 32 + lane] : 0.f;
+    int n = 0;
+#pragma unroll
+    for (int m = 0; m < kWN; ++m) {
+      v[m] = normv(v[m], st);
+      n += __popc(__ballot_sync(0xffffffffu, w0 + m * 32 + lane < a.ntime_out && v[m] > thr));
     }
+    if (lane == 0) w_s[k][warp] = n;
+    __syncthreads();  // the other buffer's readers passed the barrier before
+    int pos0 = base, round = 0;
 #pragma unroll
-    for (int m = 0; m < kWR; ++m) {
-      const int col = cs + m * kT + tid;
-      bal[m] = __ballot_sync(0xffffffffu, col < a.ntime_out && v[m] > thr);
-      if (lane == 0) w_s[m][warp] = __popc(bal[m]);
+    for (int i = 0; i < kT / 32; ++i) {
+      if (i < warp) pos0 += w_s[k][i];
+      round += w_s[k][i];
     }
-    __syncthreads();
-    int before = base, round = 0;
+    if (n)
 #pragma unroll
-    for (int m = 0; m < kWR; ++m) {
-      int pos = before;
-      for (int i = 0; i < kT / 32; ++i) {
-        if (i == warp) pos += __popc(bal[m] & ((1u << lane) - 1u));
-        const int c = w_s[m][i];
-        if (i < warp) pos += c;
-        round += c;
+      for (int m = 0; m < kWN; ++m) {
+        const int col = w0 + m * 32 + lane;
+        const unsigned bal = __ballot_sync(0xffffffffu, col < a.ntime_out && v[m] > thr);
+        const int pos = pos0 + __popc(bal & ((1u << lane) - 1u));
+        if (((bal >> lane) & 1u) && pos < B.cap) {
+          B.cand_i[pos] = make_int4(B.beam_id, r + 1, b, col);
+          B.cand_v[pos] = v[m];
+        }
+        pos0 += __popc(bal);
       }
-      const int col = cs + m * kT + tid;
-      if (((bal[m] >> lane) & 1u) && pos < B.cap) {
-        B.cand_i[pos] = make_int4(B.beam_id, r + 1, b, col);
-        B.cand_v[pos] = v[m];
-      }
-      before = base + round;
-    }
     base += round;
-    __syncthreads();
   }
 }
 
@@ -714,19 +726,14 @@ cudaError_t smooth_stats(const SmoothArgs &a, cudaStream_t s, int scale) {
   unsigned n = 0;
   if (scale) {
     k_mean_finish<<<dim3(a.nbeam, a.nw), kFin, 0, s>>>(a);
-    k_row_stat<false, true><<<dim3(a.nrows, a.nw), kT, 0, s>>>(a);
-    k_stat_finish<false, true><<<dim3(a.nbeam, a.nw), kFin, 0, s>>>(a);
-    n += 3;
+    n += 1 + row_stat<false, true>(a, a.nw, s);
   } else {
     k_stat_zero<<<a.nbeam, 32, 0, s>>>(a);
     n += 1;
   }
   if (a.w0 == 0) {  // the gate statistics of the normalised width-0 plane
-    k_row_stat<true, false><<<dim3(a.nrows, 1), kT, 0, s>>>(a);
-    k_stat_finish<true, false><<<a.nbeam, kFin, 0, s>>>(a);
-    k_row_stat<true, true><<<dim3(a.nrows, 1), kT, 0, s>>>(a);
-    k_stat_finish<true, true><<<a.nbeam, kFin, 0, s>>>(a);
-    n += 4;
+    n += row_stat<true, false>(a, 1, s);
+    n += row_stat<true, true>(a, 1, s);
   }
   count_launches(n);
   return cudaGetLastError();

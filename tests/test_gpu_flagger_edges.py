@@ -3,14 +3,15 @@ warps and rounds of blocks, short chains), bit for bit against the oracle."""
 import numpy as np
 import pytest
 
-from helpers import oracle_pipeline, small_params
+from helpers import cands_equal, oracle_pipeline, small_params
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nchan,gulp", [(32, 256), (64, 288), (96, 544), (128, 256), (160, 2080), (224, 1024),
-                                        (96, 4896), (2048, 512), (8192, 256), (32, 77856)])
-def test_flagger_edges(hella, oracle, nchan, gulp):
+@pytest.mark.parametrize("nchan,gulp,nbeam", [(32, 256, 1), (64, 288, 1), (96, 544, 1), (128, 256, 1), (160, 2080, 1),
+                                              (224, 1024, 1), (96, 4896, 1), (1024, 512, 1), (2048, 512, 1),
+                                              (8192, 256, 2), (32, 77856, 2)])
+def test_flagger_edges(hella, oracle, nchan, gulp, nbeam):
     rng = np.random.default_rng(nchan + gulp)
     x = np.clip(rng.normal(120, 25, (gulp, nchan)) + np.linspace(0, 60, nchan), 0, 255).astype(np.uint8)
     x[:, 1] = 0
@@ -19,11 +20,11 @@ def test_flagger_edges(hella, oracle, nchan, gulp):
     x[gulp // 3] = 255  # samples above and below all others
     x[gulp // 2] = 0
     s = hella.Search(hella.default_params(**small_params(nchan=nchan, gulp=gulp, df_mhz=-(468.75 - 375.0) / nchan,
-                                                         dm_max=20.0)))
-    s.load_gulp(x[None])
+                                                         dm_max=20.0, nbeam=nbeam)))
+    s.load_gulp(np.stack([x[::-1]] * (nbeam - 1) + [x]))
     s.fast_flagger()
     out, ts, tr = oracle.flag_beam(x)
-    st = s.flag_stats(0)
+    st = s.flag_stats(nbeam - 1)
 
     def same(a, b):  # bit for bit; which NaN an operation makes is not defined
         a, b = np.float32(a), np.float32(b)
@@ -33,7 +34,7 @@ def test_flagger_edges(hella, oracle, nchan, gulp):
         assert same(st[k], tr[k]), k
     assert same(st["ts"], ts)
     if not np.isnan(st["mean2"]):  # the byte of a NaN is not defined either
-        assert np.array_equal(s.copy_window(0)[-gulp:], out)
+        assert np.array_equal(s.copy_window(nbeam - 1)[-gulp:], out)
 
 
 @pytest.mark.parametrize("gulp", [256, 288, 1056, 2080, 8480])
@@ -67,3 +68,20 @@ def test_requant_every_half():
     ref = np.clip(scale * (h + np.float32(4)), 0, 255).astype(np.uint8)
     held = np.clip(h, np.float32(-4), np.float32(10.0078125)) + np.float32(4)
     assert np.array_equal(np.floor(np.float64(scale) * held).astype(np.int64) & 255, ref)
+
+
+@pytest.mark.parametrize("gulp,snr,cap", [(544, 2.0, 100000), (544, 2.0, 777), (16416, 3.0, 100000), (16416, 2.0, 5001)])
+def test_many_candidates(hella, oracle, gulp, snr, cap):
+    """Rows full of candidates, several rounds a row and more rows than a scan takes
+    at once; the cap reached within a row."""
+    p = small_params(nchan=64, gulp=gulp, df_mhz=-(468.75 - 375.0) / 64, dm_max=60.0, dm_tol=1.05, width_max=64, snr=snr,
+                     max_giants=cap, always_find_peaks=1)
+    s = hella.Search(hella.default_params(**p))
+    pl = oracle_pipeline(oracle, p)
+    rng = np.random.default_rng(gulp)
+    for g in range(pl.min_gulp + 1):
+        x = rng.integers(90, 166, (1, gulp, 64), dtype=np.uint8)
+        got, _ = s.process_gulp(x)
+        want, _ = pl.gulp_step(x)
+        assert cands_equal(got, want)
+    assert len(got) == cap or cap == 100000 and len(got) > 1000
