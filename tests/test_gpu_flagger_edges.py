@@ -85,3 +85,22 @@ def test_many_candidates(hella, oracle, gulp, snr, cap):
         want, _ = pl.gulp_step(x)
         assert cands_equal(got, want)
     assert len(got) == cap or cap == 100000 and len(got) > 1000
+
+
+@pytest.mark.parametrize("nchan,gulp,box", [(32, 288, (1, 1)), (96, 2080, (5, 3)), (160, 544, (16, 8)), (64, 1056, (2, 31))])
+def test_planes_edges(hella, oracle, nchan, gulp, box):
+    """The fp16 planes' passes at odd sizes, with and without whole batches of loads,
+    against the oracle."""
+    rng = np.random.default_rng(nchan + gulp)
+    x = np.clip(rng.normal(120, 25, (gulp, nchan)), 0, 255).astype(np.uint8)
+    x[gulp // 3:gulp // 3 + 5, 3:9] = 255
+    p = small_params(nchan=nchan, gulp=gulp, df_mhz=-(468.75 - 375.0) / nchan, dm_max=20.0)
+    entries = [(box[0], box[1], 3.0, 1)]
+    s = hella.Search(hella.default_params(**p, scrunches=entries))
+    fspec = np.zeros(nchan, np.float32)
+    s.load_gulp(x[None])
+    s.fast_flagger()
+    out, ts, _ = oracle.flag_beam(x, oracle.flag_params(scrunches=entries), fspec)
+    assert np.array_equal(s.flag_stats(0)["ts"].view(np.uint32), ts.view(np.uint32))
+    assert np.array_equal(s.copy_window(0)[-gulp:], out)
+    assert np.array_equal(s.flag_spec().view(np.uint32), fspec.view(np.uint32))
