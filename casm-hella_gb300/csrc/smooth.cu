@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kFin) k_stat_finish(SmoothArgs a) {
 // computeRowVariances over one row of one width plane.  NORM0: the
 // normalised width-0 plane (find_peaks' sigma, peaks.cu:171-178), which
 // needs width 0 in the launch (w0 == 0).  FIN: the last row's block of a (beam,
-// width) runs stat_finish.  Bound by the memory: 2286 rows x 65,536 x 9 widths 813 us
+// width) runs stat_finish.  Bound by the memory: 2499 rows x 65,536 x 9 widths 840 us
 // (6.9 TB/s).
 template <bool NORM0, bool VAR, bool FIN>
 __global__ void __launch_bounds__(kT, !NORM0 && !FIN ? 8 : 6) k_row_stat(SmoothArgs a) {
