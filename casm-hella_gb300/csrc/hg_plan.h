@@ -14,8 +14,8 @@ std::vector<float> delay_table(int nchan, double dt_s, double f0, double df);
 std::vector<int> dm_delays(const std::vector<float> &dms, const std::vector<float> &table);
 
 // Dedispersion tile tables for trials [first, first + count) with dpt
-// trials per tile (0: the largest up to dpt_max that fits cc-channel stages): host copy
-// (cached per range and shape) and device copy (uploaded on first use).
+// trials per tile (0: the largest up to dpt_max, 16, 8 or 4, that fits cc-channel stages):
+// host copy (the last range's, for each dpt_max) and device copy (uploaded on first use).
 const DedispTables &plan_host_tables(hdd_plan p, int first, int count, int dpt = 0, int cc = 8, int dpt_max = 16);
 struct DeviceTables {
   const int4 *meta;

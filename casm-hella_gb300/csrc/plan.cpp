@@ -82,14 +82,19 @@ struct hdd_plan_struct {
   std::vector<int> delays, chans;
   std::vector<hdd_bool> killmask;
   int max_delay = 0;
-  // dedispersion tile tables of the last DM range used, host and device
-  hg::DedispTables tab;
-  int tab_first = -1, tab_count = -1, tab_dpt = -1, tab_cc = -1, tab_max = -1;
-  bool tab_on_device = false;
+  // dedispersion tile tables of the last DM range used, host and device, one for
+  // each largest tile asked for (16, 8 and 4 trials): which one an execute call takes goes
+  // by its number of samples, and calls of several lengths on one DM range may be queued
+  // together
+  struct Tiles {
+    hg::DedispTables tab;
+    int first = -1, count = -1, dpt = -1, cc = -1;
+    bool on_device = false;
+    int4 *d_meta = nullptr;
+    int *d_off = nullptr;
+    size_t meta_cap = 0, off_cap = 0;
+  } tiles[3];
   int *d_err = nullptr;  // dedispersion status word
-  int4 *d_meta = nullptr;
-  int *d_off = nullptr;
-  size_t meta_cap = 0, off_cap = 0;
   uint8_t *d_in = nullptr, *d_out = nullptr;
   uint32_t *d_packed = nullptr;
   size_t in_cap = 0, out_cap = 0, packed_cap = 0;
@@ -120,8 +125,10 @@ namespace {
 thread_local int t_device = 0;
 
 void invalidate_tables(hdd_plan p) {
-  p->tab_first = p->tab_count = p->tab_dpt = p->tab_cc = -1;
-  p->tab_on_device = false;
+  for (hdd_plan_struct::Tiles &t : p->tiles) {
+    t.first = t.count = t.dpt = t.cc = -1;
+    t.on_device = false;
+  }
   p->sub_first = p->sub_count = -1;
   p->sub_on_device = false;
   p->pair_first = p->pair_count = p->pair_cc = p->pair_ntt = p->pair_g = -1;
@@ -171,42 +178,57 @@ hdd_error grow(void **ptr, size_t *cap, size_t need) {
   return HDD_NO_ERROR;
 }
 
+// Before device tables are written (`held`: they hold others): launches queued
+// earlier may still read those, and the copies are not ordered behind a
+// non-blocking stream's work.
+hdd_error settle(hdd_plan p, bool held) {
+  if (!held || !p->stream) return HDD_NO_ERROR;  // the copies run on the legacy stream themselves
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(p->stream, &cap) != cudaSuccess) return HDD_INTERNAL_GPU_ERROR;
+  if (cap != cudaStreamCaptureStatusNone) return HDD_NO_ERROR;  // recorded, not running
+  return cudaStreamSynchronize(p->stream) == cudaSuccess ? HDD_NO_ERROR : HDD_INTERNAL_GPU_ERROR;
+}
+
+hdd_plan_struct::Tiles &tile_slot(hdd_plan p, int dpt, int dpt_max) {
+  return p->tiles[dpt > 0 || dpt_max >= 16 ? 0 : dpt_max >= 8 ? 1 : 2];
+}
+
 }  // namespace
 
 namespace hg {
 
 const DedispTables &plan_host_tables(hdd_plan p, int first, int count, int dpt, int cc, int dpt_max) {
-  if (dpt > 0) dpt_max = 16;
-  if (p->tab_first != first || p->tab_count != count || p->tab_dpt != dpt || p->tab_cc != cc ||
-      p->tab_max != dpt_max) {
-    p->tab = dedisp_tables(p->delays.data(), p->nchans, p->chans.data(), (int)p->chans.size(), first,
-                           count, dpt, cc, dpt_max);
-    p->tab_max = dpt_max;
-    p->tab_first = first;
-    p->tab_count = count;
-    p->tab_dpt = dpt;
-    p->tab_cc = cc;
-    p->tab_on_device = false;
+  hdd_plan_struct::Tiles &t = tile_slot(p, dpt, dpt_max);
+  if (t.first != first || t.count != count || t.dpt != dpt || t.cc != cc) {
+    t.tab = dedisp_tables(p->delays.data(), p->nchans, p->chans.data(), (int)p->chans.size(), first, count, dpt, cc,
+                          dpt_max);
+    t.first = first;
+    t.count = count;
+    t.dpt = dpt;
+    t.cc = cc;
+    t.on_device = false;
   }
-  return p->tab;
+  return t.tab;
 }
 
 hdd_error plan_device_tables(hdd_plan p, int first, int count, DeviceTables *out, int dpt, int cc, int dpt_max) {
   const DedispTables &t = plan_host_tables(p, first, count, dpt, cc, dpt_max);
-  if (!p->tab_on_device) {
+  hdd_plan_struct::Tiles &d = tile_slot(p, dpt, dpt_max);
+  if (!d.on_device) {
     const size_t mb = std::max<size_t>(t.meta.size(), 1) * sizeof(int4);
     const size_t ob = std::max<size_t>(t.off.size(), 1) * sizeof(int);
     hdd_error e;
-    if ((e = grow((void **)&p->d_meta, &p->meta_cap, mb)) != HDD_NO_ERROR) return e;
-    if ((e = grow((void **)&p->d_off, &p->off_cap, ob)) != HDD_NO_ERROR) return e;
+    if ((e = settle(p, d.d_meta != nullptr)) != HDD_NO_ERROR) return e;
+    if ((e = grow((void **)&d.d_meta, &d.meta_cap, mb)) != HDD_NO_ERROR) return e;
+    if ((e = grow((void **)&d.d_off, &d.off_cap, ob)) != HDD_NO_ERROR) return e;
     if (!t.meta.empty() &&
-        (cudaMemcpy(p->d_meta, t.meta.data(), t.meta.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess ||
-         cudaMemcpy(p->d_off, t.off.data(), t.off.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess))
+        (cudaMemcpy(d.d_meta, t.meta.data(), t.meta.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess ||
+         cudaMemcpy(d.d_off, t.off.data(), t.off.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess))
       return HDD_MEM_COPY_FAILED;
-    p->tab_on_device = true;
+    d.on_device = true;
   }
-  out->meta = p->d_meta;
-  out->off = p->d_off;
+  out->meta = d.d_meta;
+  out->off = d.d_off;
   out->dpt = t.dpt;
   out->max_spread = t.max_spread;
   out->nact = (int)p->chans.size();
@@ -228,7 +250,8 @@ hdd_error plan_sub_tables(hdd_plan p, int first, int count, SubDeviceTables *out
   }
   const SubTables &t = p->sub;
   if (!p->sub_on_device) {
-    hdd_error e;
+    hdd_error e = settle(p, p->d_smeta != nullptr);
+    if (e != HDD_NO_ERROR) return e;
     if ((e = grow((void **)&p->d_smeta, &p->smeta_cap, std::max<size_t>(t.meta.size(), 1) * sizeof(int4))) !=
             HDD_NO_ERROR ||
         (e = grow((void **)&p->d_sindex, &p->sindex_cap, std::max<size_t>(t.index.size(), 1) * sizeof(int2))) !=
@@ -301,6 +324,7 @@ hdd_error plan_pair_tables(hdd_plan p, int first, int count, int cc, int ntt, in
   if (e != HDD_NO_ERROR) return e;
   const PairTables &t = p->pair;
   if (!p->pair_on_device) {
+    if ((e = settle(p, p->d_prinfo != nullptr)) != HDD_NO_ERROR) return e;
     auto up = [&](void **d, size_t *cap, const void *src, size_t n) -> hdd_error {
       hdd_error r = grow(d, cap, std::max<size_t>(n, 16));
       if (r != HDD_NO_ERROR) return r;
@@ -478,8 +502,10 @@ hdd_error hdd_create_plan(hdd_plan *plan, hdd_size nchans, hdd_float dt, hdd_flo
 void hdd_destroy_plan(hdd_plan p) {
   if (!p) return;
   cudaSetDevice(p->device);
-  cudaFree(p->d_meta);
-  cudaFree(p->d_off);
+  for (hdd_plan_struct::Tiles &t : p->tiles) {
+    cudaFree(t.d_meta);
+    cudaFree(t.d_off);
+  }
   cudaFree(p->d_err);
   cudaFree(p->d_in);
   cudaFree(p->d_packed);
