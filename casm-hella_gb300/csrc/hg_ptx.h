@@ -133,14 +133,14 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
 
 // Whether this block is the last of n to get here, once per launch: true in every
 // thread of that block, which then sees what the others wrote before (read it past
-// the L1).  *done is 0 before and after.  Called by a whole block.
+// the L1).  *done is 0 before and after: it wraps by itself at n, so that it comes
+// back to 0 even after launches that a caller let overlap.  Called by a whole block.
 __device__ __forceinline__ bool last_block(unsigned *done, unsigned n) {
   __shared__ bool last_s;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();  // after the barrier: all the block's writes
-    last_s = atomicAdd(done, 1u) == n - 1;
-    if (last_s) *done = 0u;
+    last_s = atomicInc(done, n - 1) == n - 1;
     __threadfence();
   }
   __syncthreads();

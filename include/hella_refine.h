@@ -17,7 +17,10 @@
  * and chi2 = sum over c, t of (d - m)^2 (unit-variance noise).
  * theta[i] = {dm (pc cm^-3), t0 (samples), width (ms), amp, index}.
  * All pointers are device pointers; work is issued on the context's
- * stream and every call returns once it is queued. */
+ * stream and every call returns once it is queued.  The calls of a context
+ * share its buffers and run one after another: a caller who gives it another
+ * stream orders that one behind the old one's work (calls that overlap all
+ * the same leave their own results undefined, not those of later calls). */
 #ifndef HELLA_REFINE_H
 #define HELLA_REFINE_H
 

@@ -92,3 +92,39 @@ def test_non_finite_samples_reach_the_results(hella, bad, steps):
     assert np.isfinite(got[0]).all() and np.isfinite(c[0])
     assert got[1, 0] == 0 and got[1, 2] == np.float32(0.05) and np.isnan(got[1, [1, 3, 4]]).all()
     assert not np.isfinite(c[1]) and (steps == 1 or np.isnan(c[1]))
+
+
+@pytest.mark.gpu
+def test_calls_after_overlapping_calls(hella):
+    """Calls of one context on two streams without an order between them leave
+    their own results undefined, never those of the calls after them."""
+    import torch
+
+    n, nchan, nsamp = 24, 1024, 512
+    r = hella.Refine(n, nchan, nsamp, TS, F0, -(468.75 - 375.0) / nchan)
+    cut = torch.randn((n, nchan, nsamp), device="cuda")
+    dm = torch.full((n,), 300.0, device="cuda")
+    theta = torch.tensor([300.2, nsamp / 2, 5.0, 0.7, 0.3], device="cuda").repeat(n, 1)
+    one = torch.ones(n, device="cuda")
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def calls():
+        chi2, grad = torch.full((n,), -1.0, device="cuda"), torch.full((n, 5), -1.0, device="cuda")
+        torch.cuda.synchronize()
+        r.forward(cut, dm, theta, chi2)
+        r.adjoint(cut, dm, theta, one, grad)
+        torch.cuda.synchronize()
+        return chi2.cpu().numpy(), grad.cpu().numpy()
+
+    chi2, grad = calls()
+    for _ in range(5):
+        outs = [(torch.empty(n, device="cuda"), torch.empty((n, 5), device="cuda")) for _ in streams]
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for s, (c, g) in zip(streams, outs):
+                r.set_stream(s.cuda_stream)
+                r.forward(cut, dm, theta, c)
+                r.adjoint(cut, dm, theta, one, g)
+        torch.cuda.synchronize()
+        after = calls()
+        assert np.array_equal(after[0], chi2) and np.array_equal(after[1], grad)
