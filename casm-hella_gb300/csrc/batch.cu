@@ -274,8 +274,11 @@ hella_status batch_sizes(const hella_batch_params *bp, hdd_plan *plan_out, Sizes
   z->ntime_dd = p.gulp + p.width_max;
   z->ntime_out = p.gulp;
   z->nbox = 0;
-  for (int sm = p.width_min; sm < p.width_max; sm *= 2) z->nbox++;
-  size_t dd_floats = 0, rows = 0, tab_bytes = 0;
+  size_t dd_floats = 0, rows = 0, tab_bytes = 0, taps = 0;
+  for (int sm = p.width_min; sm < p.width_max; sm *= 2) {
+    z->nbox++;
+    taps += (2 * (size_t)sm + 16) / 16 * 16;  // 2 sm + 1, padded to a multiple of 16
+  }
   for (int i = 0; i < nb; ++i) {
     dd_floats += (size_t)z->cap_ndms[i] * z->ntime_dd;
     rows += (size_t)z->cap_ndms[i] - 2;
@@ -284,12 +287,15 @@ hella_status batch_sizes(const hella_batch_params *bp, hdd_plan *plan_out, Sizes
   }
   const size_t R = z->R, cap = p.max_giants;
   const size_t lanes = bp->inflight == 2 ? 2 : 1;
-  z->fixed = lanes * hg::gulp_bytes(p) + (size_t)nb * nch * R * 5 + (size_t)nb * nch * 5 +
-             (size_t)nb * nch * (256 * 6 + 16) + (size_t)nb * p.gulp * 6 + dd_floats * 4 + rows * z->nbox * 20 +
+  z->fixed = lanes * hg::gulp_bytes(p) + (size_t)nb * nch * R * 5 + (size_t)nb * nch * 5 +  // plain, packed; keep, ew
+             // level tables (whole slices); part, bp1-3, rowval, flag2; ts, hts, tdiv
+             (size_t)nb * hg::lut_slices(nch) * hg::kLutSl * 512 + (size_t)nb * nch * (256 * 4 + 17) +
+             (size_t)nb * p.gulp * 14 + dd_floats * 4 + rows * (z->nbox * 20 + 4) + taps * 4 +
              (p.nscrunch > 0 || p.input_format ? (size_t)nb * nch * ((size_t)p.gulp * 6 + 8) : 0) +
              (size_t)nch * 4 +
-             (size_t)nb * cap * 20 + lanes * (size_t)nb * cap * sizeof(hella_cand) + (size_t)nb * 512 +
-             tab_bytes;
+             (size_t)nb * cap * 20 + lanes * (size_t)nb * cap * sizeof(hella_cand) +
+             // stats, counters; the other words of a slot; the words of a batch
+             (size_t)nb * z->nbox * 20 + (size_t)nb * 512 + 4096 + tab_bytes;
   z->per_width = rows * z->ntime_out * 4;
   *plan_out = plan;
   return HELLA_OK;

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import synth
-from helpers import cands_equal
+from helpers import cands_equal, small_params
 
 pytestmark = pytest.mark.gpu
 
@@ -112,3 +112,18 @@ def test_admission_by_budget(hella):
     ok.close()
     with pytest.raises(hella.HellaError, match="budget"):
         hella.Batch(hella.default_params(**dict(params, nbeam=5, hbm_budget=budget)), **kw)
+
+
+@pytest.mark.parametrize("nchan,gulp,wmax", [(32, 32768, 16), (160, 16384, 16), (128, 256, 4096), (8192, 256, 2)])
+@pytest.mark.parametrize("nbeam", [1, 7])
+def test_batch_bytes_cover_the_allocations(hella, nchan, gulp, wmax, nbeam):
+    """What a batch allocates is no more than what hella_batch_bytes says, with
+    ragged slices of channels, long gulps, many widths; and no more than the
+    budget of a batch admitted by that figure."""
+    params = small_params(nchan=nchan, nbeam=nbeam, gulp=gulp, df_mhz=-(468.75 - 375.0) / nchan, dm_max=10.0,
+                          width_max=wmax, max_giants=64)
+    said = hella.batch_bytes(hella.default_params(**params))
+    b = hella.Batch(hella.default_params(**dict(params, hbm_budget=said)))
+    held = b.info(0).device_bytes
+    b.close()
+    assert held <= said, held - said
