@@ -96,6 +96,12 @@ __device__ __forceinline__ BuildRow build_row(const DedispArgs &a, int r, bool q
 // with up to 3 words before (copies start 16-byte aligned) and rounded to whole 16 bytes.
 __host__ __device__ constexpr int build_window(int ch, int span) { return (ch + span + 6) / 4 * 4; }
 
+// Where channel i's window starts in shared memory (i = g: the words of all g).  Channel 0 is what the
+// delays are relative to and has no range of its own.
+__host__ __device__ constexpr int build_at(int i, int ch, int span) {
+  return i ? build_window(ch, 0) + (i - 1) * build_window(ch, span) : 0;
+}
+
 // One run of up to 256 packed words of a row: output word i takes bytes 0 and 2 of the packed
 // words x[c_i][i], output word i + 256 (i < n2) bytes 1 and 3, for lo <= i < hi.  NC: the group's
 // channels.  With both, the odd bytes are split off and added; the sum of the whole words, in which
@@ -170,7 +176,7 @@ __global__ void __launch_bounds__(256, G == 4 ? 4 : 5) k_pair_build(DedispArgs a
       long pos = (bm.win0 + P0 + rr.x) % R;
       if (pos < 0) pos += R;
       const int sh = (int)(pos & 3), len = (sh + kBuildCH + rr.y - rr.x + 3) / 4 * 4;
-      const int at = i * build_window(kBuildCH, a.pair_span);
+      const int at = build_at(i, kBuildCH, a.pair_span);
       off_s[i] = at + sh - rr.x;
       pos -= sh;
       mbar_arrive_tx(bar, 4u * (uint32_t)len);
@@ -727,10 +733,11 @@ cudaError_t dedisperse_pairs(const DedispArgs &a, cudaStream_t s) {
       a.pair_lanecap > pair_lanecap(g))
     return cudaErrorInvalidValue;
   if (a.R <= 0 || (!a.beams && a.one.win0 < 0)) return cudaErrorInvalidValue;
-  // the group's channel windows: ch words for c0, ch + its r range for the others
+  // the group's channel windows: ch words for c0, ch + its r range for the others, up to 200 KB of
+  // them (ranges of 43,008 samples for pairs, 14,336 for quads); the windows' alignment comes on top
   const int ch = build_chunk(g);
-  const size_t bsmem = (size_t)g * build_window(ch, a.pair_span) * 4;
-  if (bsmem > 200 * 1024) return cudaErrorInvalidValue;
+  if (((size_t)g * ch + (size_t)(g - 1) * a.pair_span) * 4 > 200 * 1024) return cudaErrorInvalidValue;
+  const size_t bsmem = (size_t)build_at(g, ch, a.pair_span) * 4;
   auto kern = g == 4 ? k_pair_build<4> : k_pair_build<2>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem);
   if (e != cudaSuccess) return e;
