@@ -1027,9 +1027,9 @@ cudaError_t launch_var(const DedispArgs &a, cudaStream_t s) {
   if (!nbuf) nbuf = 2;  // very coarse DM lists: one block per SM
   if (nbuf < 2 || nbuf > kMaxBuf) return cudaErrorInvalidValue;
   const size_t smem = smem_bytes(DPT, CC, rowstride, nbuf);
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;
+  if (smem > (size_t)kSmemMost) return cudaErrorInvalidValue;
   auto kern = k_dedisp<DPT, CC, MODE, VAR>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per_sm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
@@ -1088,8 +1088,8 @@ cudaError_t launch_sub(const DedispArgs &a, cudaStream_t s) {
   }
   if (nbuf < 2 || nbuf > kMaxBuf) return cudaErrorInvalidValue;
   const size_t smem = dedisp_sub_smem(a.max_spread, a.sub_words, a.sub_rec, nbuf);
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_dedisp_sub, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > (size_t)kSmemMost) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(k_dedisp_sub, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per_sm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -33,6 +33,11 @@ constexpr int kDedispThreads = kPackS;
 // kernel (default; the search contexts may tune it).
 constexpr int kDedispGroup = 8;
 
+// Dynamic shared memory of a block.  A kernel's limit on it belongs to the kernel, not
+// to a launch: where launches differ in size, each sets the most that any may take (a
+// limit of its own size would refuse a larger launch that another thread is making).
+constexpr int kSmemMost = 227 * 1024;
+
 // ------------------------------------------------------------- flagger
 // Channels of a slice of the flagger's level tables.
 constexpr int kLutSl = 128;

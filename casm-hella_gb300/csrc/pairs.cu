@@ -60,7 +60,7 @@ constexpr int kTileSamples = 4 * S;
 __host__ __device__ constexpr int build_chunk(int g) { return g <= 2 ? 4096 : 2048; }
 constexpr int kTmemAt = 440;              // the block's tensor memory address, in the first unit's header
 constexpr int kBarHdr = 448;              // full[4] | empty[4] | per-warp staging cursors
-constexpr size_t kSmemMost = 227 * 1024;  // of a block, one to an SM
+constexpr int kBuildMost = 200 * 1024;    // bytes of a build block's chunk and ranges, without the windows' alignment
 constexpr int kMaxBuf = 4;
 
 // Shared memory of one unit of the sum (half a block): barriers and cursors, staging buffers.
@@ -532,7 +532,7 @@ template <int CC, bool MULTI>
 cudaError_t launch_sum(const DedispArgs &a, cudaStream_t s) {
   const int bufbytes = stage_hdr_bytes(CC) + a.pair_stage;
   // the pipeline asked for, else the deepest that leaves room for two units; two buffers at least
-  const size_t share = kSmemMost / 2 / 16 * 16;
+  const size_t share = kSmemMost / 2 / 16 * 16;  // one block an SM
   int nbuf = a.nbuf;
   if (!nbuf) {
     nbuf = kMaxBuf;
@@ -548,7 +548,7 @@ cudaError_t launch_sum(const DedispArgs &a, cudaStream_t s) {
   // units per block: two where they fit, unless each item can have an SM of its own
   const int halves = one <= share && a.nitems > sms ? 2 : 1;
   auto kern = k_pair_sum<CC, MULTI>;
-  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(halves * one))) != cudaSuccess)
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost)) != cudaSuccess)
     return e;
   const int grid = std::max(1, std::min((a.nitems + halves - 1) / halves, sms));
   kern<<<grid, halves * kDedispThreads, halves * one, s>>>(a, bufbytes, nbuf);
@@ -736,10 +736,10 @@ cudaError_t dedisperse_pairs(const DedispArgs &a, cudaStream_t s) {
   // the group's channel windows: ch words for c0, ch + its r range for the others, up to 200 KB of
   // them (ranges of 43,008 samples for pairs, 14,336 for quads); the windows' alignment comes on top
   const int ch = build_chunk(g);
-  if (((size_t)g * ch + (size_t)(g - 1) * a.pair_span) * 4 > 200 * 1024) return cudaErrorInvalidValue;
+  if (((size_t)g * ch + (size_t)(g - 1) * a.pair_span) * 4 > kBuildMost) return cudaErrorInvalidValue;
   const size_t bsmem = (size_t)build_at(g, ch, a.pair_span) * 4;
   auto kern = g == 4 ? k_pair_build<4> : k_pair_build<2>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBuildMost + 1024);
   if (e != cudaSuccess) return e;
   const dim3 grid((unsigned)((a.pair_npos + ch - 1) / ch), (unsigned)a.pair_npair, (unsigned)(a.beams ? a.nbeam : 1));
   kern<<<grid, 256, bsmem, s>>>(a);

@@ -698,7 +698,7 @@ cudaError_t smooth_planes(const SmoothArgs &a, cudaStream_t s) {
   if (bs < bend) {
     const int smw = a.wmin << (bend - 1);
     const size_t smem = sizeof(float) * ((size_t)kLC + firL_taps(smw) + (size_t)firL_rows(smw) * kLPitch);
-    cudaError_t e = cudaFuncSetAttribute(k_firL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_firL, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
     if (e != cudaSuccess) return e;
     k_firL<<<dim3(a.nrows, bend - bs), kLT, smem, s>>>(a, bend);
     count_launches(1);
