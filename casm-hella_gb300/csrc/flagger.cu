@@ -581,7 +581,7 @@ __device__ __forceinline__ uint8_t requant(__half h) {
 }
 // The same bytes as the lowest of lo and hi: x is held in [-4, 10 + 1/128], whose
 // ends give 0 and 255 (NaN gives 0), and 2^23 plus the product, rounded toward zero
-// once, ends in its whole part (checked for every half: test_requant_every_half).
+// once, ends in its whole part (k_fp16_selftest compares every half on the device).
 __device__ __forceinline__ void requant2(__half2 x, uint32_t &lo, uint32_t &hi) {
   x = __hmin2(__hmax2(x, __float2half2_rn(-4.f)), __float2half2_rn(10.0078125f));
   lo = __float_as_uint(__fmaf_rz(kRequant, __fadd_rn(__low2float(x), 4.f), 8388608.f));
@@ -1085,6 +1085,15 @@ cudaError_t flag_gulp_dev(const FlagState &st, const void *gulp, uint8_t *plain,
 namespace {
 
 __global__ void k_fp16_selftest(unsigned long long *bad, unsigned int *first) {
+  auto check = [&](bool mismatch, unsigned int a, unsigned int b) {
+    if (mismatch) {
+      atomicAdd(bad, 1ull);
+      atomicCAS(first, 0xffffffffu, (a << 16) | b);
+    }
+  };
+  auto quotient = [](__half a, __half b) {  // as k_sums and k_flag_out form it
+    return div_step(__half2float(a), __half2float(b), __frcp_rn(__half2float(b)));
+  };
   const unsigned long long n = 31744ull * 31743ull;  // a in [0, 0x7c00), b in [1, 0x7c00)
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
        i += (unsigned long long)gridDim.x * blockDim.x) {
@@ -1097,10 +1106,30 @@ __global__ void k_fp16_selftest(unsigned long long *bad, unsigned int *first) {
       mismatch |= __half_as_ushort(__hadd(a, b)) != __half_as_ushort(__float2half_rn(__fadd_rn(fa, fb)));
       mismatch |= __half_as_ushort(__hmul(a, b)) != __half_as_ushort(__float2half_rn(__fmul_rn(fa, fb)));
     }
-    if (mismatch) {
-      atomicAdd(bad, 1ull);
-      atomicCAS(first, 0xffffffffu, ((unsigned int)ab << 16) | bb);
+#pragma unroll
+    for (int sg = 0; sg < 4; ++sg) {  // signs; of a zero quotient the sign may differ
+      const __half sa = sg & 1 ? __hneg(a) : a, sb = sg & 2 ? __hneg(b) : b;
+      const unsigned short q = __half_as_ushort(__float2half_rn(quotient(sa, sb))), h = __half_as_ushort(__hdiv(sa, sb));
+      mismatch |= q != h && ((q | h) & 0x7fffu) != 0;
     }
+    check(mismatch, ab, bb);
+  }
+  // zero, infinite or NaN divisors and dividends: what div_step gives is not finite (zero by infinity too);
+  // every half requantised, as either of a pair
+  const unsigned int h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h < 65536u) {
+    const __half x = __ushort_as_half((unsigned short)h);
+    const unsigned short odd[] = {0x0000, 0x8000, 0x7c00, 0xfc00, 0x7e00, 0xfe01};
+    bool mismatch = false;
+    for (int k = 0; k < 6; ++k) {
+      mismatch |= fabsf(quotient(x, __ushort_as_half(odd[k]))) <= 3.0e38f;
+      if (k > 1) mismatch |= fabsf(quotient(__ushort_as_half(odd[k]), x)) <= 3.0e38f;
+    }
+    const __half y = __ushort_as_half((unsigned short)(h ^ 0x5a5au));
+    uint32_t lo, hi;
+    requant2(__halves2half2(x, y), lo, hi);
+    mismatch |= (lo & 0xffu) != requant(x) || (hi & 0xffu) != requant(y);
+    check(mismatch, h, h);
   }
 }
 

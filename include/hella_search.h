@@ -311,8 +311,12 @@ const char *hella_status_string(hella_status s);
  * intrinsics): over every pair of positive finite binary16 values, counts
  * the cases where __hdiv differs from the correctly rounded quotient
  * (fp32 IEEE division rounded once to fp16), and likewise __hadd/__hmul on
- * a strided subset.  first_bad receives (a << 16 | b) of the first
- * mismatch.  Synchronous. */
+ * a strided subset.  The same pairs, of either sign, check the quotient that
+ * the flagger's passes form from a reciprocal against __hdiv, every half as
+ * dividend and divisor of zeros, infinities and NaN that this quotient is
+ * then not finite (those are left to __hdiv), and every half the output
+ * stage's two-at-a-time requantisation against the single one.  first_bad
+ * receives (a << 16 | b) of the first mismatch.  Synchronous. */
 hella_status hella_fp16_selftest(int device, unsigned long long *mismatches,
                                  uint32_t *first_bad);
 

@@ -104,3 +104,24 @@ def test_planes_edges(hella, oracle, nchan, gulp, box):
     assert np.array_equal(s.flag_stats(0)["ts"].view(np.uint32), ts.view(np.uint32))
     assert np.array_equal(s.copy_window(0)[-gulp:], out)
     assert np.array_equal(s.flag_spec().view(np.uint32), fspec.view(np.uint32))
+
+
+@pytest.mark.parametrize("nchan,gulp", [(64, 288), (160, 800), (128, 4128)])
+def test_zero_time_series_in_the_tail(hella, oracle, nchan, gulp):
+    """A sample whose time series is exactly 0, past the samples that the means
+    are taken over: valid statistics, and quotients that are infinite in the
+    output stage.  Levels of 96 and 160 in a checkerboard make every table value
+    0 or 2; 64 and 128, made up for in the sample after, make -1 and 1."""
+    t0 = 256 * (gulp // 256) + 4
+    x = np.where((np.arange(nchan)[None] + np.arange(gulp)[:, None]) % 2 == 0, 96, 160).astype(np.uint8)
+    even = np.arange(nchan) % 2 == 0
+    x[t0], x[t0 + 1] = np.where(even, 64, 128), np.where(even, 192, 128)
+    s = hella.Search(hella.default_params(**small_params(nchan=nchan, gulp=gulp, df_mhz=-(468.75 - 375.0) / nchan,
+                                                         dm_max=20.0)))
+    s.load_gulp(x[None])
+    s.fast_flagger()
+    out, ts, tr = oracle.flag_beam(x)
+    assert ts[t0] == 0 and tr["mean2"] == 1 and tr["std2"] == 1
+    assert np.array_equal(out[t0], np.where(even, 0, 255))
+    assert np.array_equal(s.flag_stats(0)["ts"], ts)
+    assert np.array_equal(s.copy_window(0)[-gulp:], out)
