@@ -1011,19 +1011,15 @@ cudaError_t flag_impl(const FlagState &st, const void *gulp_in, uint8_t *plain, 
 
   cudaError_t e = cudaSuccess;
   unsigned launches = 0;
-  // lane sums, the bandpass of `mode` and the tables of `stage` with it (through the
-  // median filter where bandpass_correct applies it)
+  // lane sums, the bandpass of `mode` and the tables of `stage` made with it (through
+  // the median filter where bandpass_correct applies it)
   auto bandpass = [&](bool raw, int mode, int stage) {
     if (e == cudaSuccess) e = raw ? launch_lanes<true>(st, gulp, s) : launch_lanes<false>(st, gulp, s);
     ++launches;
     const bool median = mode != 1 && st.bp_median > 1;
     if (median) launches += lane_finish(st, mode, fin_blocks, s);
-    if (stage >= 0) {
-      launch_lut(st, stage, median ? -1 : mode, s);
-      ++launches;
-    } else if (!median) {
-      launches += lane_finish(st, mode, fin_blocks, s);
-    }
+    launch_lut(st, stage, median ? -1 : mode, s);
+    ++launches;
   };
   auto normalize = [&](int which) {  // calculate_stddev: mean pass, variance pass
     if (e == cudaSuccess) e = which ? launch_rows<false, true>(st, gulp, which, s) : launch_rows<false, false>(st, gulp, which, s);

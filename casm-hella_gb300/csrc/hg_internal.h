@@ -6,7 +6,9 @@
 //   packed   u32 [nbeam][nchan][R]          word q holds samples q, q+S,
 //                                           q+2S, q+3S (S = kPackS) of the
 //                                           ring, the dedispersion operand
-//   lut      f16 [nbeam][nchan][256]        flagger value of each u8 level
+//   lut      f16 [nbeam][slice][256][128]   flagger value of each u8 level, in
+//                                           slices of 128 channels (the last
+//                                           may be part empty)
 //   dd       f32 [ndms][ntime_dd]           dedispersed sums of one beam
 //   boxes    f32 [nbox][ndms-2][ntime_out]  smoothed planes (pre-normalise)
 #pragma once

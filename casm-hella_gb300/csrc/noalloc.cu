@@ -59,7 +59,7 @@ extern "C" hdd_error hdd_execute_noalloc(hdd_plan plan, hdd_size nsamps, const h
   if (in_nbits != 8) return HDD_UNSUPPORTED_IN_NBITS;
   if (out_nbits != 32) return HDD_UNSUPPORTED_OUT_NBITS;
   if (nsamps <= (hdd_size)v.max_delay) return HDD_TOO_FEW_NSAMPS;
-  if (nsamps > (hdd_size)(65535u * 32u)) return HDD_UNKNOWN_ERROR;  // transpose grid limit, as hdd_execute_guru
+  if (nsamps > (hdd_size)(65535u * 32u)) return HDD_UNKNOWN_ERROR;  // 32 samples a row of transpose_tf's grid
   const int nout = (int)(nsamps - v.max_delay);
   if (in_stride < (hdd_size)v.nchans) return HDD_INVALID_STRIDE;
   if (out_stride % 4 != 0 || out_stride < (hdd_size)nout * 4) return HDD_INVALID_STRIDE;

@@ -664,7 +664,7 @@ hdd_error hdd_execute_guru(hdd_plan p, hdd_size nsamps, const hdd_byte *in, hdd_
   if (in_nbits != 8) return HDD_UNSUPPORTED_IN_NBITS;
   if (out_nbits != 32) return HDD_UNSUPPORTED_OUT_NBITS;
   if (nsamps <= (hdd_size)p->max_delay) return HDD_TOO_FEW_NSAMPS;
-  if (nsamps > (hdd_size)(65535u * 32u)) return HDD_UNKNOWN_ERROR;  // transpose grid limit
+  if (nsamps > (hdd_size)(65535u * 32u)) return HDD_UNKNOWN_ERROR;  // hdd_execute_noalloc's limit, for both
   const int nout = (int)(nsamps - p->max_delay);
   if (in_stride < (hdd_size)p->nchans) return HDD_INVALID_STRIDE;
   if (out_stride % 4 != 0 || out_stride < (hdd_size)nout * 4) return HDD_INVALID_STRIDE;

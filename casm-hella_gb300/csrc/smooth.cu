@@ -692,8 +692,8 @@ cudaError_t smooth_planes(const SmoothArgs &a, cudaStream_t s) {
   if (a.nrows <= 0 || a.nw <= 0) return cudaSuccess;
   if (a.ntime_out % kLO != 0) return cudaErrorInvalidValue;
   const int bend = a.w0 + a.nw;
-  // widths 1 .. 32 of a list that starts at 1 go through k_firS, every other width through k_firL
-  // (a width of 32 there: 33 taps for the staging of a chunk of its own)
+  // widths 1 .. 32 of a list that starts at 1 go through k_firS, which reads and stages a row once
+  // for all of them; every other width through k_firL
   const int bs = a.wmin == 1 ? std::max(a.w0, std::min(bend, kSW)) : a.w0;
   if (bs < bend) {
     const int smw = a.wmin << (bend - 1);

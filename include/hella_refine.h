@@ -58,10 +58,14 @@ hella_status hella_refine_forward(hella_refine *r, int n, const float *cutouts, 
 hella_status hella_refine_adjoint(hella_refine *r, int n, const float *cutouts, const float *dm_ref,
                                   const float *theta, const float *gchi2, float *gtheta);
 /* `steps` Adam steps on chi2 (betas 0.9/0.999, eps 1e-8, per-parameter
- * learning rates lr[5], host memory) updating theta in place; every step
- * is one fused forward + adjoint pass over the cutouts.  width is kept
- * >= 0.05 ms and dm >= 0.  chi2 (may be NULL) receives the chi2 of the
- * last step's starting point. */
+ * learning rates lr[5], host memory) updating theta in place.  The last
+ * step reads every element; the others read the bursts' supports, outside
+ * which the model is exactly 0 in fp32 and the gradient gains nothing, so
+ * that a sample there that is not finite acts at the last step: its
+ * cutout's theta and chi2 end as they would had it acted at every step (not
+ * finite, dm and width at their floors).  width is kept >= 0.05 ms and
+ * dm >= 0.  chi2 (may be NULL) receives the chi2 of the last step's
+ * starting point. */
 hella_status hella_refine_fit(hella_refine *r, int n, const float *cutouts, const float *dm_ref,
                               float *theta, int steps, const float *lr, float *chi2);
 
