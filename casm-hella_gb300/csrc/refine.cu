@@ -315,11 +315,14 @@ __device__ __forceinline__ void cluster_sync() {
 // which a block reaches again only after the barrier of the step between.
 // 50 steps on 64 cutouts x 1024 x 2048: 973 us (0.88-1.05 ms with the widths
 // drawn), against 6050 us for a read of every element a step and two launches.
-// Of those, 80 us are the last step's read; the other steps are bound by the
-// latency of their loads from L2 (8 us a step for up to 16 cutouts) and, from
-// about 128 cutouts on, by issue (140 instructions a channel).  Three blocks
-// an SM (80 registers): with four (64, some spilled) a step of one cutout
-// takes 9.7 us instead of 7.
+// Of those, 80 us are the last step's read (115 us on 64 cutouts).  The other
+// steps are bound by the latency of their loads from L2 (a step of all cutouts:
+// 5.0 us for one, 7.4 for 16, 8.9 for 32, 11.0 for 50) as long as all clusters
+// are resident, which eight blocks a cutout are up to about 52 cutouts; past
+// that the last ones run after the first ones' steps (14 to 17 us for 54 to 64,
+// 26 for 128).  Three blocks an SM (80 registers): with four (64, some spilled)
+// a step of one cutout, where residency does not matter, takes 9.7 us instead
+// of 7.
 constexpr int kFitCluster = 8;
 __global__ void __launch_bounds__(kWarps * 32, 3) k_refine_fit(RefineArgs a, int n, int csize, int steps, Rates ad,
                                                              float *theta, float *chi2) {
